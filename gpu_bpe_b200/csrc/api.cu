@@ -53,7 +53,16 @@ static b200bpe_status make_ctx(int device, b200bpe_ctx** out) {
     c->c.sm_count = prop.multiProcessorCount;
     c->c.cc = prop.major * 10 + prop.minor;
     cudaError_t e = cudaStreamCreateWithFlags(&c->c.stream, cudaStreamNonBlocking);
-    if (e != cudaSuccess) { delete c; set_last_error(cudaGetErrorString(e)); return B200BPE_ERR_CUDA; }
+    if (e == cudaSuccess) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        e = cudaMemPoolCreate(&c->c.pool, &props);
+        unsigned long long keep = Ctx::POOL_KEEP;
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->c.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    if (e != cudaSuccess) { b200bpe_ctx_destroy(c); set_last_error(cudaGetErrorString(e)); return B200BPE_ERR_CUDA; }
     *out = c;
     return B200BPE_OK;
 }
@@ -136,6 +145,7 @@ void b200bpe_ctx_destroy(b200bpe_ctx* c) {
     cudaSetDevice(c->c.device);
     if (c->c.comm && c->c.nccl.CommDestroy) c->c.nccl.CommDestroy(c->c.comm);
     if (c->c.stream) cudaStreamDestroy(c->c.stream);
+    if (c->c.pool) cudaMemPoolDestroy(c->c.pool);
     delete c;
 }
 

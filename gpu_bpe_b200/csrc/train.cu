@@ -12,6 +12,7 @@
 #include "train_kernels.cuh"
 #include "exchange_kernels.cuh"
 #include "peer_exchange.cuh"
+#include "word_path.cuh"
 
 namespace b200bpe {
 
@@ -156,6 +157,9 @@ struct Trainer {
     bool early_stop = false;
     uint64_t cur_n = 0;
     // timing
+    WordPath* words = nullptr;    // training on the distinct words, while by_words
+    bool by_words = false;
+    bool classic = false;         // the symbol buffers and all that goes with them are allocated
     cudaEvent_t ev_run0 = nullptr, ev_run1 = nullptr;
     double last_run_ms = 0, last_reset_ms = 0;
     std::vector<cudaEvent_t> kev;
@@ -164,6 +168,12 @@ struct Trainer {
     ~Trainer();
     b200bpe_status alloc_common();
     b200bpe_status init_state();
+    b200bpe_status init_classic();
+    bool words_eligible() const;
+    b200bpe_status run_words(uint32_t until, uint32_t start_done, uint32_t* merges_out, uint32_t* counts_out, b200bpe_progress_cb cb, void* user,
+                             std::chrono::steady_clock::time_point t0);
+    b200bpe_status run_classic(uint32_t until, uint32_t start_done, uint32_t* merges_out, uint32_t* counts_out, b200bpe_progress_cb cb, void* user,
+                               std::chrono::steady_clock::time_point t0);
     b200bpe_status build_graph();
     b200bpe_status enqueue_merge(int iter, bool timed);
     b200bpe_status grow_table();
@@ -179,8 +189,10 @@ struct Trainer {
 Trainer::~Trainer() {
     if (ctx) cudaSetDevice(ctx->device);
     if (graph) cudaGraphExecDestroy(graph);
-    if (own_inputs) { cudaFree(d_bytes); cudaFree(d_mask); }
-    cudaFree(d_sym_init);
+    if (ctx) cudaStreamSynchronize(ctx->stream);
+    delete words;
+    if (own_inputs && ctx) { ctx->free(d_bytes); ctx->free(d_mask); }
+    if (ctx) ctx->free(d_sym_init);
     cudaFree(buf[0]); cudaFree(buf[1]); cudaFree(table); cudaFree(d_state); cudaFree(d_log);
     cudaFree(d_cta_best); cudaFree(d_desc); cudaFree(d_cand); cudaFree(dq.minus); cudaFree(dq.plus); cudaFree(dq.counts);
     xch.release();
@@ -193,6 +205,7 @@ Trainer::~Trainer() {
 }
 
 b200bpe_status Trainer::alloc_common() {
+    classic = true;
     cap_elems = ((n0 + 3) & ~3ull) + 8;
     B2_CUDA(cudaMalloc(&buf[0], cap_elems * 4));
     B2_CUDA(cudaMalloc(&buf[1], cap_elems * 4));
@@ -239,8 +252,6 @@ b200bpe_status Trainer::alloc_common() {
         B2_CUDA(cudaMalloc(&dq.counts, (size_t)dq.segments * 8));
         B2_CUDA(cudaMemsetAsync(dq.counts, 0, (size_t)dq.segments * 8, ctx->stream));
     }
-    B2_CUDA(cudaEventCreate(&ev_run0));
-    B2_CUDA(cudaEventCreate(&ev_run1));
     B2_CUDA(cudaFuncSetAttribute(k_pair_count<PC_SLOTS, PC_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  PC_SMEM_BYTES));
     // The count and merge kernels need the largest shared-memory carve-out; the small kernels between them ask for
@@ -268,11 +279,54 @@ b200bpe_status Trainer::alloc_common() {
     return B200BPE_OK;
 }
 
-// Rebuild the tagged symbols from the resident inputs and put the control block back to the
-// state of a fresh BPETrainer.train call (trainer.js:187-196).
+// Which runs train on the dictionary of distinct words: "fixed" compaction on one GPU, new ids above the byte values, no option that
+// is about the other path's kernels (a recount per merge, the test of its bounded wait).  Positions are 32-bit with a bit to spare.
+bool Trainer::words_eligible() const {
+    return ctx->world == 1 && opts.compat_mode == B200BPE_COMPAT_FIXED && !(opts.flags & B200BPE_FLAG_FULL_RECOUNT) && !opts.test_first_tile &&
+           opts.first_token_id >= 256 && n0 < (1ull << 31);
+}
+
+// Puts everything back to the state of a fresh BPETrainer.train call (trainer.js:187-196), from the resident inputs.
 b200bpe_status Trainer::init_state() {
     cudaStream_t s = ctx->stream;
+    if (!ev_run0) B2_CUDA(cudaEventCreate(&ev_run0));
+    if (!ev_run1) B2_CUDA(cudaEventCreate(&ev_run1));
     B2_CUDA(cudaEventRecord(ev_run0, s));
+    merges_done = 0;
+    early_stop = false;
+    cur_n = n0;
+    std::memset(&stats, 0, sizeof(stats));
+    by_words = false;
+    if (words_eligible()) {
+        if (!words) {
+            words = new WordPath();
+            b200bpe_status r = words->create(ctx, n0, merges_goal, opts.table_log2);
+            if (r) return r;
+        }
+        const uint64_t before = words->launches;
+        b200bpe_status r = words->build(d_bytes, has_mask ? d_mask : nullptr, d_sym_init, opts.first_token_id, &by_words);
+        if (r) return r;
+        launches += words->launches - before;
+    }
+    if (!by_words) {
+        b200bpe_status r = init_classic();
+        if (r) return r;
+    }
+    B2_CUDA(cudaEventRecord(ev_run1, s));
+    B2_CUDA(cudaStreamSynchronize(s));
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ev_run0, ev_run1);
+    last_reset_ms = ms;
+    return B200BPE_OK;
+}
+
+// The symbol buffers: rebuild the tagged symbols from the resident inputs.
+b200bpe_status Trainer::init_classic() {
+    cudaStream_t s = ctx->stream;
+    if (!classic) {
+        b200bpe_status r = alloc_common();
+        if (r) return r;
+    }
     if (d_sym_init) {
         B2_CUDA(cudaMemcpyAsync(buf[0], d_sym_init, n0 * 4, cudaMemcpyDeviceToDevice, s));
     } else {
@@ -312,17 +366,7 @@ b200bpe_status Trainer::init_state() {
     h_state->cand_tau_next = 0xFFFFFFFFu;
     h_state->cand = d_cand;
     B2_CUDA(cudaMemcpyAsync(d_state, h_state, sizeof(DevState), cudaMemcpyHostToDevice, s));
-    B2_CUDA(cudaEventRecord(ev_run1, s));
-    B2_CUDA(cudaStreamSynchronize(s));
-    {
-        float ms = 0;
-        cudaEventElapsedTime(&ms, ev_run0, ev_run1);
-        last_reset_ms = ms;
-    }
-    merges_done = 0;
-    early_stop = false;
-    cur_n = n0;
-    std::memset(&stats, 0, sizeof(stats));
+    B2_CUDA(cudaStreamSynchronize(s));     // the control block's host copy is read back into next
     return B200BPE_OK;
 }
 
@@ -452,17 +496,141 @@ b200bpe_status Trainer::run(uint32_t max_merges, uint32_t* merges_out, uint32_t*
                             uint32_t* early_out, b200bpe_progress_cb cb, void* user) {
     B2_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    const bool timed = (opts.flags & B200BPE_FLAG_TIME_KERNELS) != 0;
-    const bool use_graph = !timed && !(opts.flags & B200BPE_FLAG_NO_GRAPH);
     uint32_t remaining = merges_goal - merges_done;
     if (max_merges && max_merges < remaining) remaining = max_merges;
-    const uint32_t start_done = merges_done;
-    if (timed && kev.empty()) {
-        kev.resize((size_t)(opts.batch_merges + SPARE_ITERS) * 8);
-        for (auto& e : kev) B2_CUDA(cudaEventCreate(&e));
-    }
+    const uint32_t start_done = merges_done, until = merges_done + remaining;
     auto t0 = std::chrono::steady_clock::now();
     B2_CUDA(cudaEventRecord(ev_run0, s));
+    b200bpe_status r = B200BPE_OK;
+    if (by_words) {
+        r = run_words(until, start_done, merges_out, counts_out, cb, user, t0);
+        if (r) return r;
+    }
+    if (!by_words) {
+        r = run_classic(until, start_done, merges_out, counts_out, cb, user, t0);
+        if (r) return r;
+    }
+    B2_CUDA(cudaEventRecord(ev_run1, s));
+    B2_CUDA(cudaEventSynchronize(ev_run1));
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ev_run0, ev_run1);
+    last_run_ms = ms;
+    if (n_out) *n_out = merges_done - start_done;
+    if (early_out) *early_out = early_stop ? 1u : 0u;
+    return B200BPE_OK;
+}
+
+// Batches of merges on the dictionary, a few of them enqueued ahead of the host: the control block decides on the device whether a
+// batch still has work, so one that was enqueued past an early stop is empty.
+b200bpe_status Trainer::run_words(uint32_t until, uint32_t start_done, uint32_t* merges_out, uint32_t* counts_out, b200bpe_progress_cb cb, void* user,
+                                  std::chrono::steady_clock::time_point t0) {
+    cudaStream_t s = ctx->stream;
+    WordPath& w = *words;
+    const bool timed = (opts.flags & B200BPE_FLAG_TIME_KERNELS) != 0;
+    if (timed && kev.empty()) {
+        kev.resize(2);
+        for (auto& e : kev) B2_CUDA(cudaEventCreate(&e));
+    }
+    const uint32_t ahead_most = timed ? 1 : WordPath::IN_FLIGHT;
+    uint32_t enqueued = merges_done;             // target of the last batch enqueued
+    uint32_t head = 0, tail = 0;                 // batches enqueued, batches seen
+    uint32_t targets[WordPath::IN_FLIGHT];
+    while (merges_done < until && !early_stop) {
+        while (head - tail < ahead_most && enqueued < until) {
+            const uint32_t from = enqueued, i = head % WordPath::IN_FLIGHT;
+            enqueued += std::min(opts.batch_merges, until - enqueued);
+            targets[i] = enqueued;
+            if (timed) B2_CUDA(cudaEventRecord(kev[0], s));
+            b200bpe_status r = w.enqueue_batch(enqueued);
+            if (r) return r;
+            launches++;
+            if (timed) B2_CUDA(cudaEventRecord(kev[1], s));
+            B2_CUDA(cudaMemcpyAsync(w.h_state + i, w.args.st, sizeof(WordState), cudaMemcpyDeviceToHost, s));
+            B2_CUDA(cudaMemcpyAsync(w.h_log + from, w.args.log + from, (size_t)(enqueued - from) * sizeof(uint4), cudaMemcpyDeviceToHost, s));
+            B2_CUDA(cudaEventRecord(w.ev[i], s));
+            head++;
+        }
+        const uint32_t i = tail % WordPath::IN_FLIGHT;
+        B2_CUDA(cudaEventSynchronize(w.ev[i]));
+        const WordState st = w.h_state[i];
+        tail++;
+        if (st.status & ~(uint32_t)WS_GROW) {
+            // a pair table or candidate list that filled up within one merge: run again on the symbol buffers
+            B2_CUDA(cudaStreamSynchronize(s));
+            by_words = false;
+            early_stop = false;
+            const uint32_t had = merges_done;
+            merges_done = 0;
+            cur_n = n0;
+            b200bpe_status r = init_classic();
+            if (r == B200BPE_OK && had) r = run_classic(had, 0, nullptr, nullptr, nullptr, nullptr, t0);
+            return r;
+        }
+        if (timed) {
+            float ms = 0;
+            cudaEventElapsedTime(&ms, kev[0], kev[1]);
+            stats.merge_compact_ms += ms;
+            stats.merge_compact_launches++;
+        }
+        for (uint32_t k = merges_done; k < st.merges_done; k++) {
+            const size_t o = (size_t)(k - start_done);
+            const uint4 l = w.h_log[k];
+            if (merges_out) { merges_out[o * 3 + 0] = l.x; merges_out[o * 3 + 1] = l.y; merges_out[o * 3 + 2] = l.z; }
+            if (counts_out) counts_out[o] = l.w;
+        }
+        const bool got = st.merges_done != merges_done;
+        merges_done = st.merges_done;
+        cur_n = st.symbols;
+        early_stop = st.early_stop != 0;
+        if (cb && (merges_done >= targets[i] || early_stop)) {
+            b200bpe_progress p{};
+            p.merge_index = merges_done;
+            p.total_merges = merges_goal;
+            if (got) { const uint4 l = w.h_log[merges_done - 1]; p.last_a = l.x; p.last_b = l.y; p.last_new_id = l.z; p.last_count = l.w; }
+            p.symbol_count = cur_n;
+            const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+            p.merges_per_second = el > 0 ? (merges_done - start_done) / el : 0.0;
+            cb(&p, user);
+        }
+        if (st.status == WS_GROW) {
+            // the batches behind this one found the same status and did nothing; the next ones start where this one stopped
+            b200bpe_status r = w.grow();
+            if (r) return r;
+            launches += 2;
+            tail = head;
+            enqueued = merges_done;
+            // (a batch keeps its end: progress is reported at the same merges as without the growth)
+            if (targets[i] > merges_done) {
+                const uint32_t k = head % WordPath::IN_FLIGHT;
+                const uint32_t from = merges_done;
+                enqueued = targets[k] = targets[i];
+                if (timed) B2_CUDA(cudaEventRecord(kev[0], s));
+                r = w.enqueue_batch(enqueued);
+                if (r) return r;
+                launches++;
+                if (timed) B2_CUDA(cudaEventRecord(kev[1], s));
+                B2_CUDA(cudaMemcpyAsync(w.h_state + k, w.args.st, sizeof(WordState), cudaMemcpyDeviceToHost, s));
+                B2_CUDA(cudaMemcpyAsync(w.h_log + from, w.args.log + from, (size_t)(enqueued - from) * sizeof(uint4), cudaMemcpyDeviceToHost, s));
+                B2_CUDA(cudaEventRecord(w.ev[k], s));
+                head++;
+            }
+        }
+    }
+    return B200BPE_OK;
+}
+
+// Batches of merges on the symbol buffers.
+b200bpe_status Trainer::run_classic(uint32_t until, uint32_t start_done, uint32_t* merges_out, uint32_t* counts_out, b200bpe_progress_cb cb, void* user,
+                                    std::chrono::steady_clock::time_point t0) {
+    cudaStream_t s = ctx->stream;
+    const bool timed = (opts.flags & B200BPE_FLAG_TIME_KERNELS) != 0;
+    const bool use_graph = !timed && !(opts.flags & B200BPE_FLAG_NO_GRAPH);
+    uint32_t remaining = until - merges_done;
+    if (timed && kev.size() < (size_t)(opts.batch_merges + SPARE_ITERS) * 8) {
+        for (auto& e : kev) cudaEventDestroy(e);
+        kev.assign((size_t)(opts.batch_merges + SPARE_ITERS) * 8, nullptr);
+        for (auto& e : kev) B2_CUDA(cudaEventCreate(&e));
+    }
     int grow_retries = 0, idle_batches = 0;
     uint32_t full_scans_seen = 0;
     {
@@ -611,13 +779,6 @@ b200bpe_status Trainer::run(uint32_t max_merges, uint32_t* merges_out, uint32_t*
             cb(&p, user);
         }
     }
-    B2_CUDA(cudaEventRecord(ev_run1, s));
-    B2_CUDA(cudaEventSynchronize(ev_run1));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ev_run0, ev_run1);
-    last_run_ms = ms;
-    if (n_out) *n_out = merges_done - start_done;
-    if (early_out) *early_out = early_stop ? 1u : 0u;
     return B200BPE_OK;
 }
 
@@ -658,7 +819,7 @@ static b200bpe_status make_trainer(b200bpe_ctx* c, const uint8_t* bytes, const u
     cudaStream_t s = c->c.stream;
     const size_t nb = std::max<uint64_t>(n, 1);
     if (symbols) {
-        if (cudaMalloc(&t->d_sym_init, nb * 4) != cudaSuccess) return fail(B200BPE_ERR_OOM);
+        if (c->c.alloc(&t->d_sym_init, nb * 4) != cudaSuccess) return fail(B200BPE_ERR_OOM);
         if (n && cudaMemcpyAsync(t->d_sym_init, symbols, n * 4, device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s) != cudaSuccess)
             return fail(B200BPE_ERR_CUDA);
     } else if (device_inputs) {
@@ -667,16 +828,14 @@ static b200bpe_status make_trainer(b200bpe_ctx* c, const uint8_t* bytes, const u
         t->d_mask = const_cast<uint8_t*>(mask);
         t->has_mask = mask != nullptr;
     } else {
-        if (cudaMalloc(&t->d_bytes, nb) != cudaSuccess) return fail(B200BPE_ERR_OOM);
+        if (c->c.alloc(&t->d_bytes, nb) != cudaSuccess) return fail(B200BPE_ERR_OOM);
         if (n && cudaMemcpyAsync(t->d_bytes, bytes, n, cudaMemcpyHostToDevice, s) != cudaSuccess) return fail(B200BPE_ERR_CUDA);
         if (mask) {
-            if (cudaMalloc(&t->d_mask, nb) != cudaSuccess) return fail(B200BPE_ERR_OOM);
+            if (c->c.alloc(&t->d_mask, nb) != cudaSuccess) return fail(B200BPE_ERR_OOM);
             if (n && cudaMemcpyAsync(t->d_mask, mask, n, cudaMemcpyHostToDevice, s) != cudaSuccess) return fail(B200BPE_ERR_CUDA);
             t->has_mask = true;
         }
     }
-    r = t->alloc_common();
-    if (r) return fail(r);
     r = t->init_state();
     if (r) return fail(r);
     *out = t;
@@ -733,6 +892,18 @@ b200bpe_status b200bpe_trainer_symbols(b200bpe_trainer* h, uint32_t* out, uint64
     if (!h || !n_out) return B200BPE_ERR_BAD_ARG;
     Trainer* t = h->t;
     B2_CUDA(cudaSetDevice(t->ctx->device));
+    if (t->by_words) {
+        *n_out = t->cur_n;
+        if (!out) return B200BPE_OK;
+        if (cap < t->cur_n) return B200BPE_ERR_CAPACITY;
+        uint32_t* d_out = nullptr;
+        B2_CUDA(t->ctx->alloc(&d_out, std::max<uint64_t>(1, t->cur_n) * 4));
+        b200bpe_status r = t->words->expand(d_out);
+        if (r == B200BPE_OK && cudaMemcpyAsync(out, d_out, t->cur_n * 4, cudaMemcpyDeviceToHost, t->ctx->stream) != cudaSuccess) r = B200BPE_ERR_CUDA;
+        t->ctx->free(d_out);
+        B2_CUDA(cudaStreamSynchronize(t->ctx->stream));
+        return r;
+    }
     B2_CUDA(cudaMemcpyAsync(t->h_state, t->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, t->ctx->stream));
     B2_CUDA(cudaStreamSynchronize(t->ctx->stream));
     const uint32_t e = t->h_state->epoch;
@@ -750,6 +921,24 @@ b200bpe_status b200bpe_trainer_pair_counts(b200bpe_trainer* h, uint64_t* keys_ou
     Trainer* t = h->t;
     B2_CUDA(cudaSetDevice(t->ctx->device));
     cudaStream_t s = t->ctx->stream;
+    if (t->by_words) {     // the table is always up to date: read it out
+        unsigned long long* dk = nullptr;
+        uint32_t *dc = nullptr, *dn = nullptr, nd = 0;
+        const uint32_t dcap = (uint32_t)std::min<uint64_t>(cap, 1ull << t->words->args.table_log2);
+        B2_CUDA(t->ctx->alloc(&dk, (size_t)dcap * 8));
+        B2_CUDA(t->ctx->alloc(&dc, (size_t)dcap * 4));
+        B2_CUDA(t->ctx->alloc(&dn, 4));
+        B2_CUDA(cudaMemsetAsync(dn, 0, 4, s));
+        k_word_dump<<<t->ctx->sm_count * 4, 256, 0, s>>>(t->words->args.table, t->words->args.table_log2, dk, dc, dcap, dn);
+        B2_CUDA(cudaMemcpyAsync(&nd, dn, 4, cudaMemcpyDeviceToHost, s));
+        B2_CUDA(cudaStreamSynchronize(s));
+        const uint32_t m = std::min(nd, dcap);
+        if (keys_out) B2_CUDA(cudaMemcpy(keys_out, dk, (size_t)m * 8, cudaMemcpyDeviceToHost));
+        if (counts_out) B2_CUDA(cudaMemcpy(counts_out, dc, (size_t)m * 4, cudaMemcpyDeviceToHost));
+        for (void* p : {(void*)dk, (void*)dc, (void*)dn}) t->ctx->free(p);
+        *n_distinct_out = nd;
+        return nd > cap ? B200BPE_ERR_CAPACITY : B200BPE_OK;
+    }
     B2_CUDA(cudaMemcpyAsync(t->h_state, t->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
     B2_CUDA(cudaStreamSynchronize(s));
     // An incrementally maintained table that is up to date is read out as it stands; otherwise

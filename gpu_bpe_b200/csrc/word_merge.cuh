@@ -1,0 +1,559 @@
+// The merge loop on the dictionary of word_dict.cuh: one kernel launch runs a whole batch of merges.
+//
+// What a merge has to touch is small: the occurrences of one pair among the distinct words (a few hundred late in a run), found
+// without looking at anything else, because of two facts.  An occurrence of pair (x, y) comes into being when the younger of its
+// symbols is made, so the occurrences of all pairs whose younger symbol is m are written, once, by merge m: a list of (position of
+// the left symbol, pair), and the merge that takes (x, y) reads the list of max(x, y) and keeps the entries of its own pair.
+// Byte pairs have exact lists of their own (k_dict_lists).  And a pair's count never rises after the merge that made it, so the
+// arg-max needs only the pairs above a threshold: a candidate list made by a scan of the pair table, to which a merge adds the
+// new pairs that reach the threshold; when the best candidate falls below it, the table is scanned again.
+//
+// What bounds a merge is then a chain of dependent memory round trips (occurrence list -> records -> pair table -> candidates'
+// counts), and the barriers between its two phases, not bandwidth.  So the loop runs inside ONE thread-block cluster: 16 CTAs on
+// 16 SMs, whose hardware barrier costs a fraction of a grid-wide one, with the arg-max exchanged through distributed shared
+// memory.  Against full passes over the symbol buffers (train_kernels.cuh, which "literal" compaction and sharded runs take): 64 MiB,
+// 8,000 merges 522 -> 85 ms; heavy-tailed 256 MiB, 4,000 merges 1,326 -> 77 ms; 1 GiB, 32,000 merges 16.5 -> 0.46 s.
+// Phase 1 finds and verifies the occurrences (all reads see the state before the merge), updates the pair table and
+// writes the list of the new symbol; phase 2 rewrites the records and takes the arg-max of the next merge.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "word_dict.cuh"
+
+namespace b200bpe {
+
+constexpr int WM_THREADS = 512;
+constexpr int WM_CLUSTER = 16;             // CTAs (the largest cluster the hardware takes)
+constexpr int WM_QUEUE = 6144;             // occurrences a CTA keeps in shared memory between the phases
+constexpr int WM_UNROLL = 4;               // list entries a thread has in flight
+constexpr int WM_CAND = 2048;              // candidates per CTA
+constexpr uint32_t WM_CAND_GOAL = 6000;    // candidates a scan aims at, all CTAs together
+constexpr int WM_BINS = 256;
+constexpr int WM_MAX_PROBE = 4096;
+
+// Why the loop stopped (WordState::status).
+enum : uint32_t { WS_OK = 0, WS_GROW = 1u, WS_FULL = 2u, WS_CAND = 4u };
+
+struct __align__(16) WordState {
+    unsigned long long tau;      // threshold of the candidate list, as count << 32 | ~pair; ~0 = no list
+    unsigned long long best;     // best pair of the present table, if best_valid
+    uint32_t best_valid;
+    uint32_t merges_done;
+    uint32_t next_id;
+    uint32_t early_stop;
+    uint32_t status;
+    uint32_t entries;            // list entries written so far
+    uint32_t occupied;           // pair table slots in use
+    uint32_t symbols;            // live symbols of the corpus
+    uint32_t scans;              // table scans so far (statistics)
+    uint32_t pad[3];
+};
+
+struct WordArgs {
+    uint32_t* rec;                    // the dictionary's positions
+    const uint32_t* weight;
+    const uint32_t* byte_list;        // occurrences of the byte pairs
+    const uint32_t* byte_off;
+    uint2* entries;                   // {position of the left symbol, left << 16 | right}
+    uint2* segment;                   // [symbol] = {first entry, end}
+    unsigned long long* table;        // pair << 32 | count, pair = left << 16 | right, never 0
+    uint32_t table_log2;
+    uint32_t* cand;                   // candidates between launches: [WM_CLUSTER][WM_CAND + 1], count first
+    WordState* st;
+    uint4* log;                       // {a, b, new_id, count} per merge
+};
+
+struct WordShared {
+    uint2 queue[WM_QUEUE];            // {position (~0: not an occurrence), spans}
+    uint32_t cand[WM_CAND];
+    uint32_t hist[WM_BINS];
+    unsigned long long xbest[WM_CLUSTER];
+    uint32_t xflags[WM_CLUSTER];
+    unsigned long long wbest[WM_THREADS / 32];
+    uint32_t queued, ncand, flags, inserted;
+    uint32_t c_entries, c_inserted;   // the cluster's counters: those of CTA 0 are the ones in use
+    WordState init;
+};
+
+__device__ __forceinline__ uint32_t wt_hash(uint32_t key) {
+    uint32_t x = key * 0x9E3779B1u;
+    x ^= x >> 15;
+    return x * 0x85EBCA77u;
+}
+__device__ __forceinline__ unsigned long long wt_rank(unsigned long long slot) {   // order of the arg-max: larger count, then smaller pair
+    return (slot << 32) | (uint32_t)~(uint32_t)(slot >> 32);
+}
+__device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
+    const uint32_t hi = (uint32_t)(v >> 32);
+    const uint32_t mh = __reduce_max_sync(0xFFFFFFFFu, hi);
+    const uint32_t ml = __reduce_max_sync(0xFFFFFFFFu, hi == mh ? (uint32_t)v : 0u);
+    return (unsigned long long)mh << 32 | ml;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Puts a pair with its count into the table (set-up and growth; the pair is not there yet).  False: no room.
+__device__ __forceinline__ bool wt_insert(unsigned long long* __restrict__ table, uint32_t log2, unsigned long long slot) {
+    const uint32_t mask = (1u << log2) - 1u;
+    uint32_t s = wt_hash((uint32_t)(slot >> 32)) >> (32u - log2);
+    for (int p = 0; p < WM_MAX_PROBE; p++) {
+        if (__ldcg(table + s) == 0ull && atomicCAS(table + s, 0ull, slot) == 0ull) return true;
+        s = (s + 1u) & mask;
+    }
+    return false;
+}
+// The byte pairs of the corpus, and the control block of a fresh run.
+__global__ void __launch_bounds__(256)
+k_word_init(const unsigned long long* __restrict__ bins, const DictState* __restrict__ ds, unsigned long long* __restrict__ table, uint32_t log2,
+            WordState* __restrict__ st, uint32_t first_id, uint32_t n) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;      // 65,536 threads
+    const unsigned long long v = bins[i];
+    const uint32_t pair = (i >> 8) << 16 | (i & 0xFFu);
+    if (v && !wt_insert(table, log2, (unsigned long long)pair << 32 | (uint32_t)v)) atomicOr(&st->status, (uint32_t)WS_FULL);
+    if (i == 0) {
+        st->tau = ~0ull;
+        st->next_id = first_id;
+        st->symbols = n;
+        st->occupied = ds->pairs;
+    }
+}
+// Copies the pairs that still occur into a larger table.
+__global__ void __launch_bounds__(256)
+k_word_rehash(const unsigned long long* __restrict__ from, uint32_t from_log2, unsigned long long* __restrict__ to, uint32_t to_log2, WordState* __restrict__ st) {
+    uint32_t kept = 0;
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < 1u << from_log2; i += gridDim.x * 256) {
+        const unsigned long long v = from[i];
+        if ((uint32_t)v == 0u) continue;
+        if (!wt_insert(to, to_log2, v)) atomicOr(&st->status, (uint32_t)WS_FULL);
+        kept++;
+    }
+    if (kept) atomicAdd(&st->occupied, kept);
+}
+__global__ void k_word_regrown(WordState* st) { st->status = WS_OK; st->occupied = 0u; st->tau = ~0ull; st->best_valid = 0u; }
+// Read-back of the pair counts.
+__global__ void __launch_bounds__(256)
+k_word_dump(const unsigned long long* __restrict__ table, uint32_t log2, unsigned long long* __restrict__ keys, uint32_t* __restrict__ counts, uint32_t cap,
+            uint32_t* __restrict__ n) {
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < 1u << log2; i += gridDim.x * 256) {
+        const unsigned long long v = table[i];
+        if ((uint32_t)v == 0u) continue;
+        const uint32_t k = atomicAdd(n, 1u), pair = (uint32_t)(v >> 32);
+        if (k < cap) { keys[k] = (unsigned long long)(pair >> 16) << 32 | (pair & 0xFFFFu); counts[k] = (uint32_t)v; }
+    }
+}
+
+struct WordTeam {
+    WordShared& s;
+    WordShared* lead;            // CTA 0's shared memory
+    uint32_t rank, tid;
+    cooperative_groups::cluster_group cluster;
+};
+
+// Count update of one pair.  `tau` as in WordState; a rise across it makes the slot a candidate of this CTA.
+__device__ __forceinline__ void wt_update(const WordArgs& A, WordTeam& T, uint32_t pair, uint32_t slot, unsigned long long seen, uint32_t w, bool rise,
+                                          unsigned long long tau) {
+    const uint32_t mask = (1u << A.table_log2) - 1u;
+    for (int p = 0; p < WM_MAX_PROBE; p++) {
+        if (seen == 0ull) {
+            if (!rise) break;       // a pair that occurs is in the table
+            const unsigned long long fresh = (unsigned long long)pair << 32 | w;
+            seen = atomicCAS(A.table + slot, 0ull, fresh);
+            if (seen == 0ull) {
+                atomicAdd(&T.s.inserted, 1u);
+                if (wt_rank(fresh) >= tau) {
+                    const uint32_t i = atomicAdd(&T.s.ncand, 1u);
+                    if (i < WM_CAND) T.s.cand[i] = slot; else atomicOr(&T.s.flags, (uint32_t)WS_CAND);
+                }
+                return;
+            }
+        }
+        if ((uint32_t)(seen >> 32) == pair) {
+            uint32_t* count = reinterpret_cast<uint32_t*>(A.table + slot);   // the lower half
+            if (!rise) { atomicSub(count, w); return; }
+            const uint32_t old = atomicAdd(count, w);
+            const unsigned long long low = (uint32_t)~pair;
+            if (((unsigned long long)old << 32 | low) < tau && ((unsigned long long)(old + w) << 32 | low) >= tau) {
+                const uint32_t i = atomicAdd(&T.s.ncand, 1u);
+                if (i < WM_CAND) T.s.cand[i] = slot; else atomicOr(&T.s.flags, (uint32_t)WS_CAND);
+            }
+            return;
+        }
+        slot = (slot + 1u) & mask;
+        seen = __ldcg(A.table + slot);
+    }
+    atomicOr(&T.s.flags, (uint32_t)WS_FULL);
+}
+
+// Best candidate of the cluster and the CTAs' flags; ends with the cluster barrier that also publishes phase 2's writes.
+__device__ __forceinline__ void word_argmax(const WordArgs& A, WordTeam& T, unsigned long long& best, uint32_t& flags) {
+    unsigned long long mine = 0ull;
+    const uint32_t n = min(T.s.ncand, (uint32_t)WM_CAND);
+    for (uint32_t i = T.tid; i < n; i += WM_THREADS) {
+        const unsigned long long v = __ldcg(A.table + T.s.cand[i]);
+        const unsigned long long r = (uint32_t)v ? wt_rank(v) : 0ull;
+        mine = r > mine ? r : mine;
+    }
+    mine = warp_max64(mine);
+    if ((T.tid & 31) == 0) T.s.wbest[T.tid >> 5] = mine;
+    __syncthreads();
+    if (T.tid < 32) {
+        mine = warp_max64(T.tid < WM_THREADS / 32 ? T.s.wbest[T.tid] : 0ull);
+        if (T.tid < WM_CLUSTER) {
+            WordShared* to = T.cluster.map_shared_rank(&T.s, T.tid);
+            to->xbest[T.rank] = mine;
+            to->xflags[T.rank] = T.s.flags;
+        }
+        if (T.tid == 0) T.s.queued = 0u;
+    }
+    cluster_barrier();
+    const uint32_t lane = T.tid & 31;
+    best = warp_max64(lane < WM_CLUSTER ? T.s.xbest[lane] : 0ull);
+    flags = __reduce_or_sync(0xFFFFFFFFu, lane < WM_CLUSTER ? T.s.xflags[lane] : 0u);
+}
+
+// Scan of the pair table: picks a threshold that about WM_CAND_GOAL pairs (of count 2 or more) reach and lists them.  A first
+// pass bins the counts by their leading bits (8 bins per power of two); where a single bin holds more pairs than wanted (small
+// counts: many ties) further passes split it, down to the single pair.  Every CTA takes the same decisions from CTA 0's bins.
+__device__ __noinline__ void word_scan(const WordArgs& A, WordTeam& T, unsigned long long& tau) {
+    const uint32_t slots = 1u << A.table_log2;
+    const uint32_t first = T.tid * WM_CLUSTER + T.rank;
+    unsigned long long lo = 2ull << 32, hi = ~0ull;      // ranks of the pairs still to be split: [lo, hi]
+    uint32_t above = 0;                                   // pairs known to lie above hi
+    for (int level = 0; level < 12; level++) {
+        // bins of this pass: level 0 by leading bits of the count, then linear with 2^shift ranks each
+        uint32_t shift = 0;
+        if (level) while (((hi - lo) >> shift) >= WM_BINS) shift++;
+        auto bin_of = [&](unsigned long long r) -> uint32_t {
+            if (level) return (uint32_t)((r - lo) >> shift);
+            const uint32_t c = (uint32_t)(r >> 32), e = 31u - (uint32_t)__clz((int)c);
+            return e * 8u + (e >= 3u ? (c >> (e - 3u)) & 7u : (c << (3u - e)) & 7u);
+        };
+        for (uint32_t i = T.tid; i < WM_BINS; i += WM_THREADS) T.s.hist[i] = 0u;
+        cluster_barrier();
+        uint32_t* sums = T.lead->hist;
+        for (uint32_t i = first; i < slots; i += WM_THREADS * WM_CLUSTER * 4) {
+            unsigned long long v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) { const uint32_t j = i + k * WM_THREADS * WM_CLUSTER; v[k] = j < slots ? __ldcg(A.table + j) : 0ull; }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned long long r = wt_rank(v[k]);
+                if ((uint32_t)v[k] >= 2u && r >= lo && r <= hi) atomicAdd(T.s.hist + bin_of(r), 1u);
+            }
+        }
+        __syncthreads();
+        // CTA 0's bins collect everybody's (its own are there already)
+        if (T.rank != 0) for (uint32_t i = T.tid; i < WM_BINS; i += WM_THREADS) if (T.s.hist[i]) atomicAdd(sums + i, T.s.hist[i]);
+        cluster_barrier();
+        // from the top: the lowest bin down to which the list stays within the goal
+        uint32_t total = above, bin = WM_BINS;
+        __shared__ uint32_t s_bin, s_total;
+        if (T.tid == 0) {
+            while (bin > 0) {
+                const uint32_t h = sums[bin - 1];
+                if (total + h > WM_CAND_GOAL) break;
+                total += h;
+                bin--;
+            }
+            s_bin = bin;
+            s_total = total;
+        }
+        __syncthreads();
+        bin = s_bin;
+        total = s_total;
+        cluster_barrier();          // CTA 0's bins may be cleared again
+        auto low_of = [&](uint32_t b) -> unsigned long long {
+            if (level) return lo + ((unsigned long long)b << shift);
+            const uint32_t e = b >> 3, m = b & 7u;
+            return (unsigned long long)(e >= 3u ? (8u + m) << (e - 3u) : ((8u + m) >> (3u - e))) << 32;
+        };
+        if (bin == 0) { tau = lo; break; }
+        const unsigned long long cut = low_of(bin);
+        if (total >= WM_CAND_GOAL / 8 || (level && shift == 0)) { tau = cut < lo ? lo : cut; break; }
+        // too few above the cut: split the bin below it
+        above = total;
+        const unsigned long long b_lo = low_of(bin - 1);
+        if (cut - 1 < hi && bin < WM_BINS) hi = cut - 1;
+        if (b_lo > lo) lo = b_lo;
+        tau = lo;
+    }
+    if (T.tid == 0) { T.s.ncand = 0u; T.s.flags &= ~(uint32_t)WS_CAND; }
+    __syncthreads();
+    for (uint32_t i = first; i < slots; i += WM_THREADS * WM_CLUSTER * 4) {
+        unsigned long long v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) { const uint32_t j = i + k * WM_THREADS * WM_CLUSTER; v[k] = j < slots ? __ldcg(A.table + j) : 0ull; }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if ((uint32_t)v[k] >= 2u && wt_rank(v[k]) >= tau) {
+                const uint32_t c = atomicAdd(&T.s.ncand, 1u);
+                if (c < WM_CAND) T.s.cand[c] = i + k * WM_THREADS * WM_CLUSTER; else atomicOr(&T.s.flags, (uint32_t)WS_CAND);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(WM_THREADS, 1)
+k_word_merges(WordArgs A, uint32_t target) {
+    extern __shared__ __align__(16) unsigned char wm_smem[];
+    WordShared& s = *reinterpret_cast<WordShared*>(wm_smem);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), tid = threadIdx.x, lane = tid & 31;
+    WordTeam T{s, cluster.map_shared_rank(&s, 0), rank, tid, cluster};
+    constexpr uint32_t STEP = WM_THREADS * WM_CLUSTER;
+    const uint32_t gtid = tid * WM_CLUSTER + rank;        // neighbours in a list go to different SMs
+
+    if (tid < sizeof(WordState) / 4) reinterpret_cast<uint32_t*>(&s.init)[tid] = __ldcg(reinterpret_cast<const uint32_t*>(A.st) + tid);
+    uint32_t* my_cand = A.cand + (size_t)rank * (WM_CAND + 1);
+    const uint32_t nc = min(__ldcg(my_cand), (uint32_t)WM_CAND);
+    for (uint32_t i = tid; i < nc; i += WM_THREADS) s.cand[i] = __ldcg(my_cand + 1 + i);
+    __syncthreads();
+    if (tid == 0) {
+        s.queued = 0u; s.flags = 0u; s.inserted = 0u; s.ncand = s.init.tau == ~0ull ? 0u : nc;
+        s.c_entries = s.init.entries; s.c_inserted = 0u;
+    }
+    cluster_barrier();           // also: everybody has read the control block before anybody writes it
+    uint32_t done = s.init.merges_done, next_id = s.init.next_id, symbols = s.init.symbols, scans = s.init.scans;
+    uint32_t early = s.init.early_stop, status = s.init.status;
+    unsigned long long tau = s.init.tau, best = s.init.best;
+    bool valid = s.init.best_valid != 0u;
+    uint32_t occ_most = s.init.occupied;     // upper bound of the occupied slots
+    const uint32_t occ_start = s.init.occupied;
+    const uint32_t room = (1u << A.table_log2) / 4u * 3u;
+    uint32_t flags = 0u;
+    if (early || status) return;             // the same in every CTA
+
+    while (done < target) {
+        if (!valid || best < tau || (flags & WS_CAND)) {
+            word_scan(A, T, tau);
+            scans++;
+            word_argmax(A, T, best, flags);
+            if (flags & WS_CAND) { status = WS_CAND; break; }
+            valid = true;
+        }
+        const uint32_t count = (uint32_t)(best >> 32), pair = ~(uint32_t)best;
+        if (count < 2u || next_id > TOKEN_MASK) { early = 1u; break; }
+        const uint32_t a = pair >> 16, b = pair & 0xFFFFu, fresh = next_id;
+        // the pair's occurrences
+        uint32_t beg, end;
+        const bool bytes = a < 256u && b < 256u;
+        if (bytes) { beg = __ldcg(A.byte_off + (a << 8 | b)); end = __ldcg(A.byte_off + (a << 8 | b) + 1); }
+        else { const uint2 g = __ldcg(A.segment + max(a, b)); beg = g.x; end = g.y; }
+        const uint32_t len = end - beg;
+        // a merge makes at most two new pairs per symbol in use, and per occurrence
+        const uint32_t grow = 2u * min(min(len, count), fresh + 1u);
+        if (occ_most + grow > room) {
+            occ_most = occ_start + T.lead->c_inserted;     // stable here: it changes between the two barriers of a merge
+            if (occ_most + grow > room) { status = WS_GROW; break; }
+        }
+        occ_most += grow;
+
+        // ── phase 1: occurrences, counts, the new symbol's list ──
+        auto apply = [&](uint32_t qi) {
+            const uint32_t p = s.queue[qi].x;
+            const uint32_t rp = A.rec[p], w = A.weight[p];
+            const uint32_t prev_end = (rp & WP_START) ? 0u : A.rec[p - 1];
+            bool ok = wp_sym(rp) == a;
+            const uint32_t la = wp_span(rp), q = p + la;
+            const uint32_t rq = ok ? A.rec[q] : WP_START;
+            ok = ok && !(rq & WP_START) && wp_sym(rq) == b;
+            // the left neighbour: symbol x at l
+            uint32_t l = 0u, x = 0u, rl = WP_START;
+            if (ok && !(rp & WP_START)) { l = p - wp_span(prev_end); rl = A.rec[l]; x = wp_sym(rl); }
+            if (a == b && x == a) ok = false;         // inside a run of equal symbols: its first position merges the whole run
+            uint32_t r = q + wp_span(rq), rr = ok ? A.rec[r] : WP_START;
+            if (a == b) while (ok && !(rr & WP_START) && wp_sym(rr) == a) { r += wp_span(rr); rr = A.rec[r]; }
+            const uint32_t span = r - p;
+            uint32_t y = (!ok || (rr & WP_START)) ? 0u : wp_sym(rr);
+            uint32_t right_left = b;                   // symbol on the left of the right-hand neighbour before the merge
+            uint32_t new_right = y;
+            bool left = ok && x != 0u;
+            if (a != b) {
+                // an occurrence right behind this one: the pair in between is (b, a), and becomes (new, new); the left one sees to it
+                if (y == a) {
+                    const uint32_t rz = A.rec[r + wp_span(rr)];
+                    if (!(rz & WP_START) && wp_sym(rz) == b) new_right = fresh;
+                }
+                if (left && x == b && !(rl & WP_START)) {
+                    const uint32_t ll = l - wp_span(A.rec[l - 1]);
+                    if (wp_sym(A.rec[ll]) == a) left = false;
+                }
+            }
+            const bool right = y != 0u;
+            s.queue[qi] = ok ? make_uint2(p, span | (a == b ? 0u : la << 16)) : make_uint2(~0u, 0u);
+            // room in the list of the new symbol
+            const uint32_t want = (left ? 1u : 0u) + (right ? 1u : 0u);
+            const uint32_t active = __activemask();
+            uint32_t at = 0u;
+            {
+                const uint32_t one = __ballot_sync(active, want & 1u), two = __ballot_sync(active, want & 2u);
+                const uint32_t total = __popc(one) + 2u * __popc(two);
+                if (total) {
+                    const int leader = __ffs((int)active) - 1;
+                    if ((int)lane == leader) at = atomicAdd(&T.lead->c_entries, total);
+                    at = __shfl_sync(active, at, leader);
+                    const uint32_t below = (1u << lane) - 1u;
+                    at += __popc(one & below) + 2u * __popc(two & below);
+                }
+            }
+            // the four counts that change; all first probes in flight together
+            const uint32_t k0 = x << 16 | a, k1 = x << 16 | fresh, k2 = right_left << 16 | y, k3 = fresh << 16 | new_right;
+            const uint32_t sh = 32u - A.table_log2;
+            const uint32_t s0 = wt_hash(k0) >> sh, s1 = wt_hash(k1) >> sh, s2 = wt_hash(k2) >> sh, s3 = wt_hash(k3) >> sh;
+            unsigned long long v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+            if (left) { v0 = __ldcg(A.table + s0); v1 = __ldcg(A.table + s1); }
+            if (right) { v2 = __ldcg(A.table + s2); v3 = __ldcg(A.table + s3); }
+            if (left) {
+                A.entries[at++] = make_uint2(l, k1);
+                wt_update(A, T, k0, s0, v0, w, false, tau);
+                wt_update(A, T, k1, s1, v1, w, true, tau);
+            }
+            if (right) {
+                A.entries[at] = make_uint2(p, k3);
+                wt_update(A, T, k2, s2, v2, w, false, tau);
+                wt_update(A, T, k3, s3, v3, w, true, tau);
+            }
+        };
+        // Phase 2 of one occurrence.
+        auto rewrite = [&](uint32_t qi) {
+            const uint2 o = s.queue[qi];
+            if (o.x == ~0u) return;
+            const uint32_t p = o.x, span = o.y & 0x7FFFu, e = p + span - 1u;
+            const uint32_t rp = A.rec[p];
+            if (a != b) {
+                const uint32_t q = p + (o.y >> 16);
+                if (q != e) A.rec[q] = 0u;
+            } else {
+                for (uint32_t q = p + wp_span(rp); q <= e;) {
+                    const uint32_t rq = A.rec[q];
+                    A.rec[q] = 0u;
+                    q += wp_span(rq);
+                }
+            }
+            A.rec[e] = span << 16;
+            A.rec[p] = fresh | span << 16 | (rp & WP_START);
+        };
+        // The list in rounds of WM_UNROLL entries per thread; `f` takes the queued occurrences whenever the queue could overflow, and
+        // at the end.  Returns whether the queue was emptied before the end.
+        auto walk = [&](auto&& f) -> bool {
+            bool spilled = false;
+            for (uint32_t base = 0; base < len; base += STEP * WM_UNROLL) {
+                uint32_t pos[WM_UNROLL];
+                bool hit[WM_UNROLL];
+#pragma unroll
+                for (int k = 0; k < WM_UNROLL; k++) {
+                    const uint32_t i = base + k * STEP + gtid;
+                    hit[k] = i < len;
+                    pos[k] = 0u;
+                    if (hit[k]) {
+                        if (bytes) pos[k] = __ldcg(A.byte_list + beg + i);
+                        else { const uint2 g = __ldcg(A.entries + beg + i); pos[k] = g.x; hit[k] = g.y == pair; }
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < WM_UNROLL; k++) {
+                    const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit[k]);
+                    if (m) {
+                        uint32_t at = 0u;
+                        if (lane == 0) at = atomicAdd(&s.queued, (uint32_t)__popc(m));
+                        at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(m & ((1u << lane) - 1u));
+                        if (hit[k]) s.queue[at].x = pos[k];
+                    }
+                }
+                __syncthreads();
+                const uint32_t n = s.queued;
+                const bool last = base + STEP * WM_UNROLL >= len;
+                if (!last) __syncthreads();          // everybody has read the fill before the next round adds to it
+                if (last || n + WM_THREADS * WM_UNROLL > WM_QUEUE) {
+                    for (uint32_t i = tid; i < n; i += WM_THREADS) f(i);
+                    if (!last) {
+                        spilled = true;
+                        __syncthreads();
+                        if (tid == 0) s.queued = 0u;
+                        __syncthreads();
+                    }
+                }
+            }
+            return spilled;
+        };
+        static_assert(WM_THREADS * WM_UNROLL <= WM_QUEUE, "a round fits the queue");
+        const bool spilled = walk(apply);
+        if (gtid == 0) {
+            // every occurrence of the pair itself goes
+            const uint32_t sl = wt_hash(pair) >> (32u - A.table_log2);
+            wt_update(A, T, pair, sl, __ldcg(A.table + sl), count, false, tau);
+        }
+        __syncwarp();
+        cluster_barrier();
+
+        // ── phase 2: the records; the next merge's pair ──
+        if (!spilled) {
+            const uint32_t n = s.queued;
+            for (uint32_t i = tid; i < n; i += WM_THREADS) rewrite(i);
+        } else {
+            // the queue did not hold everything: find the occurrences again (their own records are as they were in phase 1: nobody
+            // else rewrites them, and the left neighbour of a run is not part of this merge)
+            __syncthreads();
+            if (tid == 0) s.queued = 0u;
+            __syncthreads();
+            walk([&](uint32_t qi) {
+                const uint32_t p = s.queue[qi].x;
+                const uint32_t rp = A.rec[p];
+                bool ok = wp_sym(rp) == a;
+                const uint32_t la = wp_span(rp), q = p + la;
+                const uint32_t rq = ok ? A.rec[q] : WP_START;
+                ok = ok && !(rq & WP_START) && wp_sym(rq) == b;
+                uint32_t r = q + wp_span(rq);
+                if (a == b && ok) {
+                    if (!(rp & WP_START) && wp_sym(A.rec[p - wp_span(A.rec[p - 1])]) == a) ok = false;
+                    uint32_t rr = A.rec[r];
+                    while (ok && !(rr & WP_START) && wp_sym(rr) == a) { r += wp_span(rr); rr = A.rec[r]; }
+                }
+                s.queue[qi] = ok ? make_uint2(p, (r - p) | (a == b ? 0u : la << 16)) : make_uint2(~0u, 0u);
+                rewrite(qi);
+            });
+        }
+        if (gtid == 0) {
+            const uint32_t e1 = s.c_entries;
+            A.segment[fresh] = make_uint2(s.init.entries, e1);
+            s.init.entries = e1;
+            A.log[done] = make_uint4(a, b, fresh, count);
+        }
+        if (tid == 0 && s.inserted) {
+            atomicAdd(&T.lead->c_inserted, s.inserted);
+            s.inserted = 0u;
+        }
+        done++;
+        next_id++;
+        symbols -= count;
+        word_argmax(A, T, best, flags);
+        if (flags & WS_FULL) { status = WS_FULL; break; }
+    }
+    // control block and candidates for the next launch
+    cluster_barrier();
+    const uint32_t n = min(s.ncand, (uint32_t)WM_CAND);
+    for (uint32_t i = tid; i < n; i += WM_THREADS) my_cand[1 + i] = s.cand[i];
+    if (tid == 0) my_cand[0] = n;
+    if (gtid == 0) {
+        WordState o = s.init;
+        o.tau = (flags & WS_CAND) ? ~0ull : tau;
+        o.best = best;
+        o.best_valid = (valid && !(flags & WS_CAND)) ? 1u : 0u;
+        o.merges_done = done;
+        o.next_id = next_id;
+        o.early_stop = early;
+        o.status = status;
+        o.occupied = occ_start + s.c_inserted;
+        o.symbols = symbols;
+        o.scans = scans;
+        *A.st = o;
+    }
+    cluster_barrier();           // no CTA ends while its shared memory may still be read
+}
+
+}  // namespace b200bpe
