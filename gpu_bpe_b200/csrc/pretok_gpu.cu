@@ -3,7 +3,9 @@
 // decode :518-554, classify :126-134, boundaries :226-292, contractions :83-110, digit runs
 // :198-204, code-point start → first byte :499-506) for input that is well-formed UTF-8 (the last
 // character may be cut short); anything else is refused, b200bpe_pretokenize (host) takes any bytes.
-// The reference first NFC-normalises with a closed WASM library (:465): the input must be NFC.
+// The reference first NFC-normalises with a closed WASM library (:465): the input must be NFC.  The kernel says, on the way,
+// whether it surely is: nearly every text consists of code points that NFC leaves alone wherever they stand, and looking them up
+// in a bitmap costs this kernel little, where the host's check of a decoded copy was most of a call (32 MiB from and to host memory: 175 -> 10.8 ms).
 //
 // Every rule but one looks at a few code points around a position; the exception is the split of
 // digit runs every three code points counted from the start of the run, which needs the distance
@@ -13,6 +15,7 @@
 // is not all digits.
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "ctx.cuh"
 
@@ -20,6 +23,7 @@ namespace b200bpe {
 
 namespace {
 #include "unicode_classes.inc"
+#include "unicode_nfc.inc"
 }
 
 enum : uint32_t { PT_LETTER = 0, PT_DIGIT = 1, PT_WS = 2, PT_PUNCT = 3, PT_SYMBOL = 4, PT_NEWLINE = 5, PT_OTHER = 6, PT_CONT = 0xFFu };
@@ -36,6 +40,7 @@ struct ClassTables {
     const uint8_t* low;          // PT_LOW entries
     const uint32_t* ranges;      // {first, last, class} triples, sorted
     uint32_t n_ranges;
+    const uint32_t* nfc;         // a bit per code point: NFC leaves it alone wherever it stands
 };
 
 __device__ __forceinline__ uint32_t class_of(const ClassTables& t, uint32_t cp) {
@@ -66,7 +71,8 @@ __device__ __forceinline__ void pt_st(unsigned long long* p, unsigned long long 
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// desc: (tag << 34) | (flag << 32) | (all_digits << 31) | digits; status[0]: 1 = malformed UTF-8, 2 = look-back timed out
+// desc: (tag << 34) | (flag << 32) | (all_digits << 31) | digits; status[0]: 1 = malformed UTF-8, 2 = look-back timed out;
+// status[1]: 1 = perhaps not in NFC, or not strictly well-formed (overlong, cut short, a surrogate)
 __global__ void __launch_bounds__(PT_THREADS)
 k_pretokenize(ClassTables tab, const uint8_t* __restrict__ bytes, uint64_t n, uint8_t* __restrict__ out,
               unsigned long long* __restrict__ desc, uint32_t* __restrict__ ticket, uint32_t* __restrict__ status,
@@ -90,7 +96,7 @@ k_pretokenize(ClassTables tab, const uint8_t* __restrict__ bytes, uint64_t n, ui
         }
         __syncthreads();
         // classes: decode wherever a code point starts (pre_tokenizer.mjs:518-554; bytes past the end read as 0)
-        bool bad = false;
+        bool bad = false, doubt = false;
         for (int i = threadIdx.x; i < PT_BEFORE + PT_TILE + PT_AFTER; i += PT_THREADS) {
             const long long g = t0 - PT_BEFORE + i;
             uint32_t cls = PT_CONT;
@@ -111,6 +117,10 @@ k_pretokenize(ClassTables tab, const uint8_t* __restrict__ bytes, uint64_t n, ui
                             const bool cont = (at((int)k) & 0xC0u) == 0x80u;
                             if (cont != (k < size)) bad = true;
                         }
+                        if (size > 1u) {
+                            const uint32_t least = size == 2u ? 0x80u : size == 3u ? 0x800u : 0x10000u;
+                            doubt |= v < least || v > 0x10FFFFu || (uint64_t)g + size > n || !((__ldg(tab.nfc + (min(v, 0x10FFFFu) >> 5)) >> (v & 31u)) & 1u);
+                        }
                     }
                     cls = class_of(tab, v);
                 } else if (g == 0) {
@@ -120,6 +130,7 @@ k_pretokenize(ClassTables tab, const uint8_t* __restrict__ bytes, uint64_t n, ui
             sc[i] = (uint8_t)cls;
         }
         if (bad) atomicExch(status, 1u);
+        if (doubt) status[1] = 1u;
         __syncthreads();
         // digit runs: per thread (digits at the end of my 16 bytes, all my code points are digits)
         const int base = PT_BEFORE + threadIdx.x * PT_PER;
@@ -284,7 +295,7 @@ k_pretokenize(ClassTables tab, const uint8_t* __restrict__ bytes, uint64_t n, ui
 }
 
 // class tables on the device, once per GPU
-struct DeviceTables { uint8_t* low = nullptr; uint32_t* ranges = nullptr; uint32_t n = 0; };
+struct DeviceTables { uint8_t* low = nullptr; uint32_t *ranges = nullptr, *nfc = nullptr; uint32_t n = 0; };
 static DeviceTables g_tables[64];
 static std::mutex g_tables_mutex;
 
@@ -292,7 +303,7 @@ static b200bpe_status tables_for(int device, ClassTables* out) {
     if (device < 0 || device >= 64) return B200BPE_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lock(g_tables_mutex);
     DeviceTables& t = g_tables[device];
-    if (!t.low) {
+    if (!t.nfc) {
         const uint32_t nr = (uint32_t)(sizeof(kClassRanges) / sizeof(kClassRanges[0]));
         std::string low(PT_LOW, (char)PT_OTHER);
         for (uint32_t r = 0; r < nr; r++)
@@ -302,8 +313,15 @@ static b200bpe_status tables_for(int device, ClassTables* out) {
         B2_CUDA(cudaMemcpy(t.low, low.data(), PT_LOW, cudaMemcpyHostToDevice));
         B2_CUDA(cudaMemcpy(t.ranges, kClassRanges, sizeof(kClassRanges), cudaMemcpyHostToDevice));
         t.n = nr;
+        std::vector<uint32_t> nfc(0x110000 / 32, 0xFFFFFFFFu);
+        for (const auto& r : kNfcDoubtful)
+            for (uint32_t cp = r[0]; cp <= r[1]; cp++) nfc[cp >> 5] &= ~(1u << (cp & 31u));
+        uint32_t* d = nullptr;
+        B2_CUDA(cudaMalloc(&d, nfc.size() * 4));
+        B2_CUDA(cudaMemcpy(d, nfc.data(), nfc.size() * 4, cudaMemcpyHostToDevice));
+        t.nfc = d;
     }
-    out->low = t.low; out->ranges = t.ranges; out->n_ranges = t.n;
+    out->low = t.low; out->ranges = t.ranges; out->n_ranges = t.n; out->nfc = t.nfc;
     return B200BPE_OK;
 }
 
@@ -317,62 +335,73 @@ b200bpe_status b200bpe_pretokenize_device(b200bpe_ctx* c, const uint8_t* d_bytes
     return b200bpe_pretokenize_device_ex(c, d_bytes, n, d_word_starts_out, 0u);
 }
 
-b200bpe_status b200bpe_pretokenize_device_ex(b200bpe_ctx* c, const uint8_t* d_bytes, uint64_t n, uint8_t* d_word_starts_out,
-                                             uint32_t test_lookback_spins) {
-    if (!c || ((!d_bytes || !d_word_starts_out) && n)) return B200BPE_ERR_BAD_ARG;
-    if (n == 0) return B200BPE_OK;
-    B2_CUDA(cudaSetDevice(c->c.device));
+// Working storage comes from the context's pool.  surely_nfc (may be null): 1 if the text is strictly well-formed and in NFC for sure.
+static b200bpe_status pretokenize(b200bpe_ctx* c, const uint8_t* d_bytes, uint64_t n, uint8_t* d_word_starts_out, uint32_t test_lookback_spins,
+                                  uint32_t* surely_nfc) {
     cudaStream_t s = c->c.stream;
     ClassTables tab{};
     b200bpe_status r = tables_for(c->c.device, &tab);
     if (r) return r;
     const uint64_t ntiles = (n + PT_TILE - 1) / PT_TILE;
-    unsigned long long* desc = nullptr;
-    uint32_t* ctl = nullptr;   // ticket, status
-    B2_CUDA(cudaMalloc(&desc, ntiles * 8));
-    if (cudaMalloc(&ctl, 8) != cudaSuccess) { cudaFree(desc); return B200BPE_ERR_OOM; }
-    uint32_t h_ctl[2] = {0, 0};
-    cudaMemsetAsync(desc, 0, ntiles * 8, s);
-    cudaMemsetAsync(ctl, 0, 8, s);
+    unsigned long long* desc = nullptr;   // two words of control (ticket, status, doubt, -), then the look-back descriptors
+    if (c->c.alloc(&desc, (ntiles + 2) * 8) != cudaSuccess) { cudaGetLastError(); return B200BPE_ERR_OOM; }
+    uint32_t* ctl = reinterpret_cast<uint32_t*>(desc);
+    uint32_t h_ctl[4] = {0, 0, 0, 0};
+    cudaMemsetAsync(desc, 0, (ntiles + 2) * 8, s);
     const bool stall = test_lookback_spins != 0u && test_lookback_spins < (1u << 20);
     if (stall) {   // the tile ticket starts at 1: tile 0 is never worked on and never publishes its digits
         static const uint32_t one = 1u;
         cudaMemcpyAsync(ctl, &one, 4, cudaMemcpyHostToDevice, s);
     }
     const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)c->c.sm_count * 8);
-    k_pretokenize<<<grid, PT_THREADS, 0, s>>>(tab, d_bytes, n, d_word_starts_out, desc, ctl, ctl + 1, 1u,
+    k_pretokenize<<<grid, PT_THREADS, 0, s>>>(tab, d_bytes, n, d_word_starts_out, desc + 2, ctl, ctl + 1, 1u,
                                               test_lookback_spins ? test_lookback_spins : PT_MAX_SPINS);
-    cudaError_t e = cudaMemcpyAsync(h_ctl, ctl, 8, cudaMemcpyDeviceToHost, s);
+    cudaError_t e = cudaMemcpyAsync(h_ctl, ctl, 16, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(desc);
-    cudaFree(ctl);
+    c->c.free(desc);
     if (e != cudaSuccess) { set_last_error(std::string("b200bpe_pretokenize_device: ") + cudaGetErrorString(e)); return B200BPE_ERR_CUDA; }
     if (h_ctl[1] == 2u) return B200BPE_ERR_LOOKBACK_TIMEOUT;
     if (h_ctl[1] == 1u) {
         set_last_error("b200bpe_pretokenize_device: the input is not well-formed UTF-8 (the host function b200bpe_pretokenize takes any bytes)");
         return B200BPE_ERR_BAD_ARG;
     }
+    if (surely_nfc) *surely_nfc = h_ctl[2] == 0u ? 1u : 0u;
     return B200BPE_OK;
 }
 
+b200bpe_status b200bpe_pretokenize_device_ex(b200bpe_ctx* c, const uint8_t* d_bytes, uint64_t n, uint8_t* d_word_starts_out,
+                                             uint32_t test_lookback_spins) {
+    if (!c || ((!d_bytes || !d_word_starts_out) && n)) return B200BPE_ERR_BAD_ARG;
+    if (n == 0) return B200BPE_OK;
+    B2_CUDA(cudaSetDevice(c->c.device));
+    return pretokenize(c, d_bytes, n, d_word_starts_out, test_lookback_spins, nullptr);
+}
+
 b200bpe_status b200bpe_pretokenize_gpu(b200bpe_ctx* c, const uint8_t* bytes, uint64_t n, uint8_t* word_starts_out) {
+    return b200bpe_pretokenize_gpu_nfc(c, bytes, n, word_starts_out, nullptr);
+}
+
+b200bpe_status b200bpe_pretokenize_gpu_nfc(b200bpe_ctx* c, const uint8_t* bytes, uint64_t n, uint8_t* word_starts_out, uint32_t* surely_nfc) {
     if (!c || ((!bytes || !word_starts_out) && n)) return B200BPE_ERR_BAD_ARG;
+    if (surely_nfc) *surely_nfc = n == 0 ? 1u : 0u;
     if (n == 0) return B200BPE_OK;
     B2_CUDA(cudaSetDevice(c->c.device));
     cudaStream_t s = c->c.stream;
     uint8_t *d_in = nullptr, *d_out = nullptr;
-    B2_CUDA(cudaMalloc(&d_in, n));
-    if (cudaMalloc(&d_out, n) != cudaSuccess) { cudaFree(d_in); return B200BPE_ERR_OOM; }
+    if (c->c.alloc(&d_in, n) != cudaSuccess) { cudaGetLastError(); return B200BPE_ERR_OOM; }
+    if (c->c.alloc(&d_out, n) != cudaSuccess) { cudaGetLastError(); c->c.free(d_in); return B200BPE_ERR_OOM; }
     cudaMemcpyAsync(d_in, bytes, n, cudaMemcpyHostToDevice, s);
-    b200bpe_status r = b200bpe_pretokenize_device(c, d_in, n, d_out);
+    uint32_t surely = 0u;
+    b200bpe_status r = pretokenize(c, d_in, n, d_out, 0u, &surely);
     cudaError_t e = cudaSuccess;
-    if (r == B200BPE_OK) {
+    if (r == B200BPE_OK && (!surely_nfc || surely)) {   // (who asks has no use for the starts of a text that has to be normalised first)
         e = cudaMemcpyAsync(word_starts_out, d_out, n, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
-    cudaFree(d_in);
-    cudaFree(d_out);
+    c->c.free(d_in);
+    c->c.free(d_out);
     if (e != cudaSuccess) { set_last_error(std::string("b200bpe_pretokenize_gpu: ") + cudaGetErrorString(e)); return B200BPE_ERR_CUDA; }
+    if (surely_nfc) *surely_nfc = surely;
     return r;
 }
 

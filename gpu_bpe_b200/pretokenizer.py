@@ -6,6 +6,7 @@ that step and the boundary rules run in the library's host code (b200bpe_pretoke
 """
 from __future__ import annotations
 
+import ctypes as C
 import unicodedata
 
 import numpy as np
@@ -25,6 +26,12 @@ class PreTokenizer:
         arr = np.frombuffer(raw, dtype=np.uint8) if not isinstance(raw, np.ndarray) else np.ascontiguousarray(raw, np.uint8)
         if arr.size == 0:
             return {"bytes": np.zeros(0, np.uint8), "wordStarts": np.zeros(0, np.uint8)}
+        if self.normalize and self.engine is not None:
+            # the device says of nearly every text that it is in NFC already; the others, and whatever it refuses, go the general way
+            mask, nfc = np.empty(arr.size, np.uint8), C.c_uint32()
+            st = _lib.lib().b200bpe_pretokenize_gpu_nfc(self.engine.ctx, arr.ctypes.data, arr.size, mask.ctypes.data, C.byref(nfc))
+            if st == 0 and nfc.value:
+                return {"bytes": arr, "wordStarts": mask}
         if self.normalize:
             try:
                 text = arr.tobytes().decode("utf-8")

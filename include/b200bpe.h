@@ -269,6 +269,9 @@ b200bpe_status b200bpe_pretokenize(const uint8_t* bytes, uint64_t n, uint8_t* wo
  * across tiles by a decoupled look-back scan. */
 b200bpe_status b200bpe_pretokenize_device(b200bpe_ctx*, const uint8_t* d_bytes, uint64_t n, uint8_t* d_word_starts_out);
 b200bpe_status b200bpe_pretokenize_gpu(b200bpe_ctx*, const uint8_t* bytes, uint64_t n, uint8_t* word_starts_out);
+/* The same for a caller who would normalise first: *surely_nfc is 1 if the text is strictly well-formed UTF-8 and NFC would leave
+ * it as it is (the quick check of UAX #15 over code points of combining class 0).  0: perhaps not; word_starts_out is then not written. */
+b200bpe_status b200bpe_pretokenize_gpu_nfc(b200bpe_ctx*, const uint8_t* bytes, uint64_t n, uint8_t* word_starts_out, uint32_t* surely_nfc);
 /* Tests only (no counterpart in the reference): the device function with the number of polls after which its
  * look-back gives up (0 = default).  A value below 2^20 also makes the kernel skip tile 0, whose digit count no
  * other tile can then obtain: the call ends with B200BPE_ERR_LOOKBACK_TIMEOUT, which proves that the wait is bounded. */
