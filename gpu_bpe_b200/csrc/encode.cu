@@ -28,6 +28,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.cuh"
@@ -402,6 +403,46 @@ __device__ __forceinline__ void st_d64(unsigned long long* p, unsigned long long
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// Tokens of the tiles before `tile`, by decoupled look-back; called by one whole warp.  The tile's own count goes out first.
+// A wait that runs out sets ctl[1] and gives 0.
+__device__ __forceinline__ unsigned long long sc_look_back(unsigned long long* __restrict__ desc, uint64_t tile, unsigned long long agg, int lane,
+                                                           uint32_t max_spins, uint32_t* __restrict__ ctl) {
+    unsigned long long excl = 0ull;
+    if (tile == 0) {
+        if (lane == 0) st_d64(desc, (2ull << 62) | agg);
+    } else {
+        if (lane == 0) st_d64(desc + tile, (1ull << 62) | agg);
+        long long pos = (long long)tile - 1;
+        uint32_t spins = 0;
+        bool timed_out = false;
+        for (;;) {
+            const long long idx = pos - lane;
+            unsigned long long d = 2ull << 62;  // before tile 0: a zero prefix
+            for (;;) {
+                if (idx >= 0) d = ld_d64(desc + idx);
+                if (__all_sync(0xFFFFFFFFu, (d >> 62) != 0ull)) break;
+                if (++spins > max_spins) { timed_out = true; break; }
+                __nanosleep(40);
+            }
+            if (timed_out) break;
+            const uint32_t pmask = __ballot_sync(0xFFFFFFFFu, (d >> 62) == 2ull);
+            const int first = pmask ? (__ffs(pmask) - 1) : 32;
+            unsigned long long contrib = (lane <= first) ? (d & 0x3FFFFFFFFFFFFFFFull) : 0ull;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xFFFFFFFFu, contrib, o);
+            excl += contrib;
+            if (pmask) break;
+            pos -= 32;
+        }
+        if (timed_out) {
+            if (lane == 0) atomicExch(&ctl[1], 1u);
+            excl = 0ull;
+        }
+        if (lane == 0) st_d64(desc + tile, (2ull << 62) | (excl + agg));
+    }
+    return excl;
+}
+
 // One tile = SC_THREADS chunks.  Sum the tile's token counts, learn the tile's offset by
 // decoupled look-back, then copy every chunk's run from its stride-`cs` staging slot to its final
 // place with coalesced warp copies.  ctl[0] = tile ticket, ctl[1] = error flag; total → *total_out.
@@ -451,39 +492,7 @@ k_scan_compact(const uint32_t* __restrict__ staging, const uint32_t* __restrict_
             }
             if (lane < SC_THREADS / 32) wsum[lane] = wi - w;
             const unsigned long long agg = __shfl_sync(0xFFFFFFFFu, wi, SC_THREADS / 32 - 1);
-            unsigned long long excl = 0ull;
-            if (tile == 0) {
-                if (lane == 0) st_d64(desc, (2ull << 62) | agg);
-            } else {
-                if (lane == 0) st_d64(desc + tile, (1ull << 62) | agg);
-                long long pos = (long long)tile - 1;
-                uint32_t spins = 0;
-                bool timed_out = false;
-                for (;;) {
-                    const long long idx = pos - lane;
-                    unsigned long long d = 2ull << 62;  // before tile 0: a zero prefix
-                    for (;;) {
-                        if (idx >= 0) d = ld_d64(desc + idx);
-                        if (__all_sync(0xFFFFFFFFu, (d >> 62) != 0ull)) break;
-                        if (++spins > max_spins) { timed_out = true; break; }
-                        __nanosleep(40);
-                    }
-                    if (timed_out) break;
-                    const uint32_t pmask = __ballot_sync(0xFFFFFFFFu, (d >> 62) == 2ull);
-                    const int first = pmask ? (__ffs(pmask) - 1) : 32;
-                    unsigned long long contrib = (lane <= first) ? (d & 0x3FFFFFFFFFFFFFFFull) : 0ull;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xFFFFFFFFu, contrib, o);
-                    excl += contrib;
-                    if (pmask) break;
-                    pos -= 32;
-                }
-                if (timed_out) {
-                    if (lane == 0) atomicExch(&ctl[1], 1u);
-                    excl = 0ull;
-                }
-                if (lane == 0) st_d64(desc + tile, (2ull << 62) | (excl + agg));
-            }
+            const unsigned long long excl = sc_look_back(desc, tile, agg, lane, max_spins, ctl);
             if (lane == 0) {
                 s_base = excl;
                 if (tile == ntiles - 1) {
@@ -514,6 +523,229 @@ k_scan_compact(const uint32_t* __restrict__ staging, const uint32_t* __restrict_
                 if (i + 64 < cnt && o + i + 64 < cap) out[o + i + 64] = v2;
                 if (i + 96 < cnt && o + i + 96 < cap) out[o + i + 96] = v3;
             }
+        }
+    }
+}
+
+// ── walks split at every 32 bytes ──
+// The walks above go through a chunk from its start, one thread each: a serial chain of some hundred steps, during which a small
+// input leaves most of the chip idle (4 MiB in chunks of 512 bytes: 8,192 threads, of the 227,000 that fit).  Greedy matching forgets
+// where it began: two walks that meet at the start of a token agree from there on, and from any two places of a text they meet
+// within a few tokens.  So here every 32-byte block of a chunk is walked by a thread of its own:
+//   1  from the block's first byte as if a token began there, noting the token of every start (all but block 0's may be wrong at first)
+//   2  on into the next blocks until a start that their own thread has noted: from there on both agree (at most 64 bytes far)
+//   3  one thread per chunk follows block to block from start 0, which is right: the true starts of a block are those noted from
+//      the place where the walk enters it, and those that phase 2 found on the way.  Where phase 2 gave up (texts like "aaaa", whose walks
+//      never meet) it walks on itself, which is then the serial chain again.
+// Ranks of the starts by a scan, the tile's place by decoupled look-back, and the tokens go out in order: no staging, no second kernel.
+// What bounds it is the chain of dependent look-ups of a block (some 30 steps) and, from some 10 MiB on, their number, a third more than
+// the walks above make.  Walk and compaction, us, before -> after, 512-byte chunks: vocabulary of 4,096 (cuckoo) 2 KiB 141 -> 28, 1 MiB
+// 487 -> 46, 4 MiB 488 -> 51, 32 MiB 523 -> 267; of 32,256 (hybrid) 2 KiB 224 -> 58, 1 MiB 537 -> 69, 4 MiB 547 -> 80, 32 MiB 587 -> 491.
+constexpr uint32_t WS_BLOCK = 32;
+constexpr uint32_t WS_REACH = 64;                 // bytes behind its block that a thread's phase 2 looks for a common start
+constexpr uint32_t WS_STRIDE = WS_BLOCK + 1;      // 16-bit tokens per block in shared memory (odd: blocks start in different banks)
+constexpr uint32_t WS_MAX_TOKEN = 0xFFFFu;
+
+template <int THREADS>
+struct SplitShared {
+    unsigned long long extra[THREADS];            // per block: starts found by phase 2, bit k = k bytes behind the block (before that,
+                                                  // per chunk of the tile: first byte)
+    uint32_t len[THREADS];
+    uint32_t noted[THREADS], real[THREADS];       // per block: starts of its own walk, true starts
+    uint32_t base[THREADS / 32];
+    uint16_t met[THREADS];                        // per block: where phase 2 stopped (relative to the chunk)
+    uint16_t token[THREADS * WS_STRIDE];
+    uint32_t tile;
+    uint64_t offset;
+};
+
+// Longest match at p (relative to the chunk at `text`, `len` bytes): its token, and p moves behind it.  D as in k_trie_walk, 1: hybrid.
+template <int D>
+__device__ __forceinline__ uint32_t longest_match(const TrieHybrid& th, const TrieDev& td, const unsigned char* smem, const uint8_t* __restrict__ text,
+                                                  uint32_t len, uint32_t& p) {
+    const uint32_t first = __ldg(text + p);
+    uint32_t w = p + 1u, next = w < len ? __ldg(text + w) : 0u;
+    uint32_t tok = first, end = w;
+    if constexpr (D == 1) {
+        const uint32_t* sm = reinterpret_cast<const uint32_t*>(smem);
+        const uint2* hot0 = reinterpret_cast<const uint2*>(sm);
+        const uint2* hot1 = hot0 + (1u << HY_BUCKET_LOG2);
+        const uint32_t n1 = sm[HY_HOT_WORDS + first];
+        tok = (n1 & HY_INDEX) <= th.max_token ? n1 & HY_INDEX : first;
+        uint32_t key = ((HY_ROOT2 | first) << 8) | next, v = 0u;
+        while (w < len) {
+            const uint32_t ahead = w + 1u < len ? __ldg(text + w + 1u) : 0u;
+            const uint32_t h0 = (key * th.mul[0]) & HY_KEY_MASK, h1 = (key * th.mul[1]) & HY_KEY_MASK;
+            const uint2 e0 = hot0[h0 >> HY_REM_SHIFT], e1 = hot1[h1 >> HY_REM_SHIFT];
+            const uint32_t r0 = h0 & ((1u << HY_REM_SHIFT) - 1u), r1 = h1 & ((1u << HY_REM_SHIFT) - 1u);
+            uint32_t nv = T_MISS;
+            nv = (e0.x >> 19) == r0 ? e0.x : nv;
+            nv = (e0.y >> 19) == r0 ? e0.y : nv;
+            nv = (e1.x >> 19) == r1 ? e1.x : nv;
+            nv = (e1.y >> 19) == r1 ? e1.y : nv;
+            bool hit = (nv & HY_INDEX) != HY_INDEX;     // an empty entry is all ones
+            if (!hit && (v & HY_COLD)) {                // (v is 0 on the two-byte first step)
+                const uint32_t hh = key * 0x9E3779B1u;
+                uint32_t slot = (hh ^ (hh >> 15)) & th.cold_mask;
+                for (;;) {
+                    const uint2 e = __ldg(th.cold + slot);
+                    if (e.x == key) { nv = e.y; hit = true; break; }
+                    if (e.x == T_EMPTY_KEY) break;
+                    slot = (slot + 1) & th.cold_mask;
+                }
+            }
+            if (!hit) break;
+            w++;
+            v = nv;
+            if ((nv & HY_INDEX) <= th.max_token) { tok = nv & HY_INDEX; end = w; }
+            if (nv & HY_LEAF) break;
+            key = ((nv & HY_INDEX) << 8) | ahead;
+        }
+    } else {
+        const uint32_t* ck = reinterpret_cast<const uint32_t*>(smem);
+        const uint32_t ck_shift = 24u - td.ck_log2, ck_rmask = (1u << ck_shift) - 1u, ck_size = 1u << td.ck_log2;
+        uint32_t key = ((td.root & CK_INDEX) << 8) | first;
+        w = p;
+        for (;;) {
+            uint32_t nv = T_MISS;
+#pragma unroll
+            for (int d = D - 1; d >= 0; d--) {
+                const uint32_t h = (key * td.ck_mul[d]) & 0xFFFFFFu;
+                const uint32_t e = ck[d * ck_size + (h >> ck_shift)];
+                nv = (e >> 18) == (h & ck_rmask) ? (e & CK_VALUE) : nv;
+            }
+            if (nv == T_MISS) break;
+            w++;
+            if (nv & CK_HAS_TOKEN) { tok = nv & CK_INDEX; end = w; }
+            if ((nv & CK_LEAF) || w >= len) break;
+            key = ((nv & CK_INDEX) << 8) | next;
+            next = w + 1u < len ? __ldg(text + w + 1u) : 0u;
+        }
+    }
+    p = end;
+    return tok;
+}
+
+// per_chunk: blocks a chunk can have; a tile is THREADS / per_chunk chunks.  The rest as in k_trie_walk and k_scan_compact.
+template <int D, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+k_trie_split(TrieHybrid th, TrieDev td, const uint8_t* __restrict__ bytes, uint64_t n, uint32_t cs, uint32_t per_chunk, const uint64_t* __restrict__ doc_off,
+             const uint64_t* __restrict__ chunk_base, uint32_t n_docs, uint64_t n_chunks_static, unsigned long long* __restrict__ desc,
+             uint32_t* __restrict__ ctl, uint64_t* __restrict__ chunk_offsets, uint32_t* __restrict__ out, uint64_t cap, uint64_t* __restrict__ total_out,
+             uint32_t max_spins) {
+    extern __shared__ __align__(16) unsigned char tw_smem[];
+    const uint32_t table_bytes = D == 1 ? HY_SMEM_BYTES : ((uint32_t)D << td.ck_log2) * 4u;
+    SplitShared<THREADS>& s = *reinterpret_cast<SplitShared<THREADS>*>(tw_smem + table_bytes);
+    const uint64_t n_chunks = chunk_base ? chunk_base[n_docs] : n_chunks_static;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (n_chunks == 0) {
+        if (blockIdx.x == 0 && tid == 0) {
+            *total_out = 0;
+            if (chunk_offsets) chunk_offsets[0] = 0;
+        }
+        return;
+    }
+    {
+        const uint4* __restrict__ src = reinterpret_cast<const uint4*>(D == 1 ? th.hot : td.cuckoo);
+        for (uint32_t i = tid; i < table_bytes / 16u; i += THREADS) reinterpret_cast<uint4*>(tw_smem)[i] = __ldg(src + i);
+    }
+    const uint32_t per_tile = THREADS / per_chunk;
+    const uint64_t ntiles = (n_chunks + per_tile - 1) / per_tile;
+    const uint32_t c = tid / per_chunk, j = tid - c * per_chunk;      // this thread's chunk of the tile, and block of that chunk
+    const uint32_t u0 = tid - j;                                      // the chunk's first block
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s.tile = atomicAdd(&ctl[0], 1u);
+        __syncthreads();
+        const uint64_t tile = s.tile;
+        if (tile >= ntiles) return;
+        if (tid < per_tile) {
+            const uint64_t g = tile * per_tile + tid;
+            uint64_t lo = 0, hi = 0;
+            if (g < n_chunks) chunk_span(g, cs, n, doc_off, chunk_base, n_docs, &lo, &hi);
+            s.extra[tid] = lo;
+            s.len[tid] = (uint32_t)(hi - lo);
+        }
+        __syncthreads();
+        const bool mine = c < per_tile;
+        const uint32_t len = mine ? s.len[c] : 0u;
+        const uint8_t* __restrict__ text = bytes + (mine ? s.extra[c] : 0ull);
+        const uint32_t lo = j * WS_BLOCK, hi = min(lo + WS_BLOCK, len);
+        auto place = [&](uint32_t p) { return (u0 + p / WS_BLOCK) * WS_STRIDE + p % WS_BLOCK; };
+        auto noted_at = [&](uint32_t p) { return (s.noted[u0 + p / WS_BLOCK] >> (p % WS_BLOCK)) & 1u; };
+        // 1: the block on its own
+        uint32_t p = lo, noted = 0u;
+        while (p < hi) {
+            const uint32_t q = p;
+            s.token[place(q)] = (uint16_t)longest_match<D>(th, td, tw_smem, text, len, p);
+            noted |= 1u << (q - lo);
+        }
+        s.noted[tid] = noted;
+        s.real[tid] = 0u;
+        __syncthreads();
+        // 2: on to a start that another block has noted
+        unsigned long long extra = 0ull;
+        if (lo < hi) {
+            while (p < len && p < hi + WS_REACH && !noted_at(p)) {
+                const uint32_t q = p;
+                s.token[place(q)] = (uint16_t)longest_match<D>(th, td, tw_smem, text, len, p);
+                extra |= 1ull << (q - hi);
+            }
+        }
+        s.extra[tid] = extra;
+        s.met[tid] = (uint16_t)p;
+        __syncthreads();
+        // 3: the true starts
+        if (mine && j == 0u && len) {
+            uint32_t b = 0u, from = 0u;
+            for (;;) {
+                const uint32_t u = u0 + b;
+                s.real[u] |= s.noted[u] & (0xFFFFFFFFu << from);
+                const unsigned long long e = s.extra[u];
+                if ((uint32_t)e) s.real[u + 1] |= (uint32_t)e;
+                if ((uint32_t)(e >> 32)) s.real[u + 2] |= (uint32_t)(e >> 32);
+                uint32_t q = s.met[u];
+                while (q < len && !noted_at(q)) {
+                    const uint32_t at = q;
+                    s.token[place(at)] = (uint16_t)longest_match<D>(th, td, tw_smem, text, len, q);
+                    s.real[u0 + at / WS_BLOCK] |= 1u << (at % WS_BLOCK);
+                }
+                if (q >= len) break;
+                b = q / WS_BLOCK;
+                from = q % WS_BLOCK;
+            }
+        }
+        __syncthreads();
+        const uint32_t real = s.real[tid], cnt = (uint32_t)__popc(real);
+        uint32_t inc = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= (uint32_t)o) inc += x;
+        }
+        if (lane == 31) s.base[warp] = inc;
+        __syncthreads();
+        uint32_t off = inc - cnt, total = 0u;
+#pragma unroll
+        for (uint32_t w = 0; w < THREADS / 32; w++) { const uint32_t v = s.base[w]; if (w < warp) off += v; total += v; }
+        if (warp == 0) {
+            const unsigned long long excl = sc_look_back(desc, tile, total, (int)lane, max_spins, ctl);
+            if (lane == 0) {
+                s.offset = excl;
+                if (tile == ntiles - 1) {
+                    *total_out = excl + total;
+                    if (chunk_offsets) chunk_offsets[n_chunks] = excl + total;
+                }
+            }
+        }
+        __syncthreads();
+        const uint64_t base = s.offset;
+        if (chunk_offsets && mine && j == 0u && tile * per_tile + c < n_chunks) chunk_offsets[tile * per_tile + c] = base + off;
+        // a warp's 32 blocks, one after the other: the starts of a block are neighbours in the output
+        for (uint32_t r = 0; r < 32; r++) {
+            const uint32_t m = __shfl_sync(0xFFFFFFFFu, real, r), at = __shfl_sync(0xFFFFFFFFu, off, r);
+            const uint64_t o = base + at + __popc(m & ((1u << lane) - 1u));
+            if (((m >> lane) & 1u) && o < cap) out[o] = s.token[(warp * 32u + r) * WS_STRIDE + lane];
         }
     }
 }
@@ -552,9 +784,9 @@ struct Tokenizer {
     uint64_t* d_doc_off = nullptr; uint64_t doc_off_cap = 0;
     uint64_t* d_chunk_base = nullptr; uint64_t chunk_base_cap = 0;
     uint64_t* d_tok_off = nullptr; uint64_t tok_off_cap = 0;
+    // {total, tile ticket | error flag << 32, chunk ticket, -}, then the look-back descriptors: one memset, one read-back per launch
     unsigned long long* d_desc = nullptr; uint64_t desc_cap = 0;
-    uint32_t* d_ctl = nullptr;
-    uint64_t* d_total = nullptr;
+    static constexpr uint64_t CTL_WORDS = 4;
     uint64_t* h_total = nullptr;  // pinned: total, error flag
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     double walk_ms = 0, compact_ms = 0;
@@ -563,7 +795,7 @@ struct Tokenizer {
         if (ctx) cudaSetDevice(ctx->device);
         cudaFree(d_trans); cudaFree(d_cuckoo); cudaFree(d_hot); cudaFree(d_cold); cudaFree(d_in); cudaFree(d_staging);
         cudaFree(d_counts); cudaFree(d_chunk_off); cudaFree(d_out); cudaFree(d_doc_off); cudaFree(d_chunk_base);
-        cudaFree(d_tok_off); cudaFree(d_desc); cudaFree(d_ctl); cudaFree(d_total);
+        cudaFree(d_tok_off); cudaFree(d_desc);
         if (h_total) cudaFreeHost(h_total);
         if (h_slices) cudaFreeHost(h_slices);
         for (auto e : ev) if (e) cudaEventDestroy(e);
@@ -588,13 +820,13 @@ struct Tokenizer {
         return B200BPE_OK;
     }
 
-    b200bpe_status ensure_work(uint64_t max_chunks) {
+    b200bpe_status ensure_work(uint64_t max_chunks, bool staging) {
         b200bpe_status r;
-        if ((r = ensure(&d_staging, &staging_cap, max_chunks * chunk))) return r;
+        if (staging && (r = ensure(&d_staging, &staging_cap, max_chunks * chunk))) return r;
         if ((r = ensure(&d_counts, &counts_cap, max_chunks + 1))) return r;
         if ((r = ensure(&d_chunk_off, &chunk_off_cap, max_chunks + 1))) return r;
-        if ((r = ensure(&d_desc, &desc_cap, max_chunks / SC_THREADS + 2))) return r;
-        return B200BPE_OK;
+        // (a tile of the split walk holds one chunk at least)
+        return ensure(&d_desc, &desc_cap, CTL_WORDS + max_chunks + 2);
     }
 
     size_t walk_smem() const { return hybrid ? (size_t)HY_SMEM_BYTES : ck_d == 0 ? (size_t)TW_SMEM_BYTES : ((size_t)ck_d << ck_log2) * 4; }
@@ -624,6 +856,56 @@ struct Tokenizer {
         }
     }
 
+    // Walks split at every 32 bytes (k_trie_split): a tile takes whole chunks, a thread per block.  512 threads, or 1,024 where only
+    // one CTA fits an SM anyway.
+    uint32_t blocks_per_chunk() const { return (chunk + WS_BLOCK - 1) / WS_BLOCK; }
+    uint32_t split_threads() const {
+        const size_t t = walk_smem();
+        return !hybrid && t + sizeof(SplitShared<512>) > 113u * 1024 && t + sizeof(SplitShared<1024>) <= 227u * 1024 ? 1024u : 512u;
+    }
+    // For tries that fit shared memory beside the tile, with 16-bit tokens, and chunks that fit a tile.
+    // A walk of whole chunks takes about 1 us per byte of a chunk while their number fits the chip; this one takes about 38 us (cuckoo) or
+    // 60 us (hybrid) per 151,552 blocks, however full they are.  It pays while  blocks x that  <  bytes per chunk:  up to 55 and 38 MB in
+    // chunks of 512 bytes (measured: level at 64 MiB and 38 MB), less in many short documents.
+    bool split_pays(uint64_t n, uint64_t max_chunks) const {
+        if ((ck_d == 0 && !hybrid) || max_token > WS_MAX_TOKEN || blocks_per_chunk() > 512u) return false;
+        if (walk_smem() + sizeof(SplitShared<512>) > 227u * 1024) return false;
+        return max_chunks * blocks_per_chunk() / 1024 * max_chunks < (hybrid ? 2400ull : 3600ull) * (n / 1024 + 1);
+    }
+    template <class F>
+    void for_split(F&& f) const {   // f(layout, threads), as types
+        using std::integral_constant;
+        if (split_threads() == 1024u) {
+            if (ck_d == 2) f(integral_constant<int, 2>{}, integral_constant<int, 1024>{});
+            else f(integral_constant<int, 3>{}, integral_constant<int, 1024>{});
+        } else if (hybrid) f(integral_constant<int, 1>{}, integral_constant<int, 512>{});
+        else if (ck_d == 2) f(integral_constant<int, 2>{}, integral_constant<int, 512>{});
+        else f(integral_constant<int, 3>{}, integral_constant<int, 512>{});
+    }
+    // The shared memory that the split walk of this trie asks for (at creation: later launches find the kernel loaded).
+    cudaError_t prepare_split() const {
+        cudaError_t e = cudaSuccess;
+        if ((ck_d == 0 && !hybrid) || walk_smem() + sizeof(SplitShared<512>) > 227u * 1024) return e;
+        for_split([&](auto d, auto threads) {
+            constexpr int D = decltype(d)::value, T = decltype(threads)::value;
+            e = cudaFuncSetAttribute(k_trie_split<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(walk_smem() + sizeof(SplitShared<T>)));
+        });
+        return e;
+    }
+    void walk_split(const uint8_t* d_bytes, uint64_t n, const uint64_t* d_docs, const uint64_t* cb, uint32_t n_docs, uint64_t ntiles,
+                    unsigned long long* desc, uint32_t* ctl, uint32_t* d_tokens, uint64_t cap, uint64_t* d_total) {
+        const TrieDev td{d_trans, trans_mask, d_cuckoo, ck_log2, {ck_mul[0], ck_mul[1], ck_mul[2]}, root};
+        const TrieHybrid th{d_hot, {hy_mul[0], hy_mul[1]}, d_cold, cold_mask, max_token};
+        for_split([&](auto d, auto threads) {
+            constexpr int D = decltype(d)::value, T = decltype(threads)::value;
+            const size_t smem = walk_smem() + sizeof(SplitShared<T>);
+            const uint64_t most = (uint64_t)ctx->sm_count * std::max<size_t>(1, 228u * 1024 / (smem + 1024));
+            k_trie_split<D, T><<<(int)std::max<uint64_t>(1, std::min<uint64_t>(most, ntiles)), T, smem, ctx->stream>>>(
+                th, td, d_bytes, n, chunk, blocks_per_chunk(), d_docs, cb, n_docs, (n + chunk - 1) / chunk, desc, ctl, d_chunk_off, d_tokens, cap,
+                d_total, sc_max_spins);
+        });
+    }
+
     // Walk + scan/compact on device-resident inputs.  d_docs == nullptr → one buffer.
     // h_dst / evs: where this launch's {total, error flag} and its three timing events go (default:
     // the tokenizer's own), so that several launches can be in flight on the stream.
@@ -635,11 +917,14 @@ struct Tokenizer {
         cudaEvent_t* ev = evs ? evs : this->ev;
         if (ck_d == 0 && !hybrid) set_persisting_window(ctx, d_trans, trans_bytes);  // keep the transition table resident in L2
         const uint64_t max_chunks = (n + chunk - 1) / chunk + (d_docs ? n_docs : 0);
-        b200bpe_status r = ensure_work(std::max<uint64_t>(1, max_chunks));
+        const bool split = split_pays(n, max_chunks);
+        b200bpe_status r = ensure_work(std::max<uint64_t>(1, max_chunks), !split);
         if (r) return r;
-        const uint64_t ntiles = max_chunks / SC_THREADS + 2;
-        B2_CUDA(cudaMemsetAsync(d_desc, 0, ntiles * 8, s));
-        B2_CUDA(cudaMemsetAsync(d_ctl, 0, 16, s));
+        const uint64_t ntiles = max_chunks / (split ? split_threads() / blocks_per_chunk() : SC_THREADS) + 2;
+        uint64_t* d_total = reinterpret_cast<uint64_t*>(d_desc);
+        uint32_t* d_ctl = reinterpret_cast<uint32_t*>(d_desc + 1);
+        unsigned long long* desc = d_desc + CTL_WORDS;
+        B2_CUDA(cudaMemsetAsync(d_desc, 0, (CTL_WORDS + ntiles) * 8, s));
         if (skip_first_tile) {   // the tile ticket starts at 1
             static const uint32_t one = 1u;
             B2_CUDA(cudaMemcpyAsync(d_ctl, &one, 4, cudaMemcpyHostToDevice, s));
@@ -651,16 +936,20 @@ struct Tokenizer {
             cb = d_chunk_base;
         }
         B2_CUDA(cudaEventRecord(ev[0], s));
-        walk(d_bytes, n, d_docs, cb, n_docs, max_chunks, d_staging, d_counts, d_ctl + 2);
-        B2_CUDA(cudaEventRecord(ev[1], s));
-        const int grid_c = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sm_count * 8, ntiles));
-        k_scan_compact<<<grid_c, SC_THREADS, 0, s>>>(d_staging, d_counts, chunk, cb, n_docs, (n + chunk - 1) / chunk, d_desc,
-                                                    d_ctl, d_chunk_off, d_tokens, cap, d_total, sc_max_spins);
+        if (split) {
+            walk_split(d_bytes, n, d_docs, cb, n_docs, ntiles, desc, d_ctl, d_tokens, cap, d_total);
+            B2_CUDA(cudaEventRecord(ev[1], s));
+        } else {
+            walk(d_bytes, n, d_docs, cb, n_docs, max_chunks, d_staging, d_counts, d_ctl + 2);
+            B2_CUDA(cudaEventRecord(ev[1], s));
+            const int grid_c = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sm_count * 8, ntiles));
+            k_scan_compact<<<grid_c, SC_THREADS, 0, s>>>(d_staging, d_counts, chunk, cb, n_docs, (n + chunk - 1) / chunk, desc,
+                                                        d_ctl, d_chunk_off, d_tokens, cap, d_total, sc_max_spins);
+        }
         B2_CUDA(cudaEventRecord(ev[2], s));
         if (d_docs && d_tok_offsets)
             k_doc_token_offsets<<<std::max(1u, std::min(1024u, (n_docs + 256) / 256)), 256, 0, s>>>(cb, d_chunk_off, n_docs, d_tok_offsets);
-        B2_CUDA(cudaMemcpyAsync(hd, d_total, 8, cudaMemcpyDeviceToHost, s));
-        B2_CUDA(cudaMemcpyAsync(hd + 1, d_ctl, 8, cudaMemcpyDeviceToHost, s));
+        B2_CUDA(cudaMemcpyAsync(hd, d_total, 16, cudaMemcpyDeviceToHost, s));
         B2_CUDA(cudaGetLastError());
         return B200BPE_OK;
     }
@@ -1065,8 +1354,7 @@ b200bpe_status b200bpe_tokenizer_create_ex(b200bpe_ctx* c, const void* trie, siz
                                         (int)(cuckoo.size() * 4)));
         }
     }
-    B2_TRY(cudaMalloc(&t->d_ctl, 16));
-    B2_TRY(cudaMalloc(&t->d_total, 8));
+    B2_TRY(t->prepare_split());
     B2_TRY(cudaMallocHost(&t->h_total, 16));
     for (auto& e : t->ev) B2_TRY(cudaEventCreate(&e));
     {
@@ -1192,14 +1480,17 @@ b200bpe_status b200bpe_encode_batch(b200bpe_tok* h, const uint8_t* bytes, const 
     std::vector<uint64_t> rel((size_t)n_docs + n_slices);
     uint64_t max_chunks = 1;
     uint32_t max_docs = 1;
+    bool staging = false;
     for (uint32_t i = 0; i < n_slices; i++) {
         const uint32_t d0 = cut[i], d1 = cut[i + 1];
         for (uint32_t d = d0; d <= d1; d++) rel[(size_t)d + i] = doc_offsets[d] - doc_offsets[d0];
-        max_chunks = std::max<uint64_t>(max_chunks, (doc_offsets[d1] - doc_offsets[d0] + t->chunk - 1) / t->chunk + (d1 - d0));
+        const uint64_t nb = doc_offsets[d1] - doc_offsets[d0], chunks = (nb + t->chunk - 1) / t->chunk + (d1 - d0);
+        max_chunks = std::max<uint64_t>(max_chunks, chunks);
+        staging |= !t->split_pays(nb, chunks);
         max_docs = std::max(max_docs, d1 - d0);
     }
     // every buffer a slice needs exists before the first one starts (growing one synchronises the stream)
-    if ((r = t->ensure_work(max_chunks))) return r;
+    if ((r = t->ensure_work(max_chunks, staging))) return r;
     if ((r = t->ensure(&t->d_chunk_base, &t->chunk_base_cap, (uint64_t)max_docs + 1))) return r;
     if ((r = t->ensure_slices(n_slices))) return r;
     B2_CUDA(cudaMemcpyAsync(t->d_doc_off, rel.data(), rel.size() * 8, cudaMemcpyHostToDevice, s));
