@@ -70,10 +70,25 @@ constexpr double HY_MAX_LOAD = 0.86;
 struct TrieHybrid {
     const uint32_t* hot;     // two sub-tables of (1 << HY_BUCKET_LOG2) buckets of two entries, then the 256 root children
     uint32_t mul[2];         // odd multipliers of the two hash functions (modulo 2^25)
-    const uint2* cold;       // open addressing: {key, value in the 4-byte entry's value format}
+    const uint4* cold;       // buckets of two {key, value in the 4-byte entry's value format}
     uint32_t cold_mask;
     uint32_t max_token;      // indices up to this one end a token
 };
+
+// The child of a node in the global table (T_MISS: none).  A dependent load from L2 is what a step of the walk waits for longest, so
+// the table is at most a quarter full and a bucket of two entries is one load: nearly every look-up, hit or miss, is a single one.
+// 32,256 entries, walk of 256 MiB 1,961 -> 1,707 us, of 4 MiB 77.6 -> 69.9 us, against single entries at half load.
+__device__ __forceinline__ uint32_t cold_child(const TrieHybrid& t, uint32_t key) {
+    const uint32_t h = key * 0x9E3779B1u;
+    uint32_t b = (h ^ (h >> 15)) & t.cold_mask;
+    for (;;) {
+        const uint4 e = __ldg(t.cold + b);
+        if (e.x == key) return e.y;
+        if (e.z == key) return e.w;
+        if (e.z == T_EMPTY_KEY) return T_MISS;     // (the first entry of a bucket fills first)
+        b = (b + 1u) & t.cold_mask;
+    }
+}
 
 struct TrieDev {
     const uint2* trans;      // {parent << 8 | byte, packed child}
@@ -324,16 +339,8 @@ k_trie_walk_hybrid(TrieHybrid t, const uint8_t* __restrict__ bytes, uint64_t n, 
             bool hit = (nv & HY_INDEX) != HY_INDEX && (two || !fresh);   // an empty entry is all ones
             if (!hit && !fresh && (v & HY_COLD)) {
                 // some of this node's children live in the global table only
-                {
-                    const uint32_t hh = key * 0x9E3779B1u;
-                    uint32_t slot = (hh ^ (hh >> 15)) & t.cold_mask;
-                    for (;;) {
-                        const uint2 e = __ldg(t.cold + slot);
-                        if (e.x == key) { nv = e.y; hit = true; break; }
-                        if (e.x == T_EMPTY_KEY) break;
-                        slot = (slot + 1) & t.cold_mask;
-                    }
-                }
+                nv = cold_child(t, key);
+                hit = nv != T_MISS;
             }
             if (fresh) {   // what the first byte alone is worth
                 have = (n1 & HY_INDEX) <= t.max_token;   // T_MISS has an index above every token id
@@ -540,7 +547,7 @@ k_scan_compact(const uint32_t* __restrict__ staging, const uint32_t* __restrict_
 // Ranks of the starts by a scan, the tile's place by decoupled look-back, and the tokens go out in order: no staging, no second kernel.
 // What bounds it is the chain of dependent look-ups of a block (some 30 steps) and, from some 10 MiB on, their number, a third more than
 // the walks above make.  Walk and compaction, us, before -> after, 512-byte chunks: vocabulary of 4,096 (cuckoo) 2 KiB 141 -> 28, 1 MiB
-// 487 -> 46, 4 MiB 488 -> 51, 32 MiB 523 -> 267; of 32,256 (hybrid) 2 KiB 224 -> 58, 1 MiB 537 -> 69, 4 MiB 547 -> 80, 32 MiB 587 -> 491.
+// 487 -> 46, 4 MiB 488 -> 51, 32 MiB 523 -> 267; of 32,256 (hybrid) 2 KiB 224 -> 53, 1 MiB 537 -> 63, 4 MiB 547 -> 73, 32 MiB 587 -> 439.
 constexpr uint32_t WS_BLOCK = 32;
 constexpr uint32_t WS_REACH = 64;                 // bytes behind its block that a thread's phase 2 looks for a common start
 constexpr uint32_t WS_STRIDE = WS_BLOCK + 1;      // 16-bit tokens per block in shared memory (odd: blocks start in different banks)
@@ -585,14 +592,8 @@ __device__ __forceinline__ uint32_t longest_match(const TrieHybrid& th, const Tr
             nv = (e1.y >> 19) == r1 ? e1.y : nv;
             bool hit = (nv & HY_INDEX) != HY_INDEX;     // an empty entry is all ones
             if (!hit && (v & HY_COLD)) {                // (v is 0 on the two-byte first step)
-                const uint32_t hh = key * 0x9E3779B1u;
-                uint32_t slot = (hh ^ (hh >> 15)) & th.cold_mask;
-                for (;;) {
-                    const uint2 e = __ldg(th.cold + slot);
-                    if (e.x == key) { nv = e.y; hit = true; break; }
-                    if (e.x == T_EMPTY_KEY) break;
-                    slot = (slot + 1) & th.cold_mask;
-                }
+                nv = cold_child(th, key);
+                hit = nv != T_MISS;
             }
             if (!hit) break;
             w++;
@@ -838,7 +839,7 @@ struct Tokenizer {
         TrieDev t{d_trans, trans_mask, d_cuckoo, ck_log2, {ck_mul[0], ck_mul[1], ck_mul[2]}, root};
         const uint64_t n_static = (n + chunk - 1) / chunk;
         if (hybrid) {
-            TrieHybrid th{d_hot, {hy_mul[0], hy_mul[1]}, d_cold, cold_mask, max_token};
+            TrieHybrid th{d_hot, {hy_mul[0], hy_mul[1]}, reinterpret_cast<const uint4*>(d_cold), cold_mask, max_token};
             const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sm_count * HY_CTAS, (max_chunks + HY_THREADS - 1) / HY_THREADS));
             k_trie_walk_hybrid<<<grid, HY_THREADS, HY_SMEM_BYTES, s>>>(th, d_bytes, n, chunk, d_docs, cb, n_docs, n_static, staging, counts, ticket);
         } else if (ck_d == 0) {
@@ -895,7 +896,7 @@ struct Tokenizer {
     void walk_split(const uint8_t* d_bytes, uint64_t n, const uint64_t* d_docs, const uint64_t* cb, uint32_t n_docs, uint64_t ntiles,
                     unsigned long long* desc, uint32_t* ctl, uint32_t* d_tokens, uint64_t cap, uint64_t* d_total) {
         const TrieDev td{d_trans, trans_mask, d_cuckoo, ck_log2, {ck_mul[0], ck_mul[1], ck_mul[2]}, root};
-        const TrieHybrid th{d_hot, {hy_mul[0], hy_mul[1]}, d_cold, cold_mask, max_token};
+        const TrieHybrid th{d_hot, {hy_mul[0], hy_mul[1]}, reinterpret_cast<const uint4*>(d_cold), cold_mask, max_token};
         for_split([&](auto d, auto threads) {
             constexpr int D = decltype(d)::value, T = decltype(threads)::value;
             const size_t smem = walk_smem() + sizeof(SplitShared<T>);
@@ -1268,15 +1269,15 @@ b200bpe_status b200bpe_tokenizer_create_ex(b200bpe_ctx* c, const void* trie, siz
             size_t n_cold = 0;
             for (size_t i = 0; i < deep.size(); i++) n_cold += in_hot[i] ? 0 : 1;
             uint32_t clog = 4;
-            while ((1ull << clog) < (uint64_t)n_cold * 2 + 16) clog++;
+            while ((1ull << clog) < (uint64_t)n_cold * 4 + 16) clog++;
             cold.assign((size_t)1 << clog, make_uint2(T_EMPTY_KEY, 0u));
-            cold_mask = (1u << clog) - 1;
+            cold_mask = (1u << (clog - 1)) - 1;       // buckets of two
             cold_bits.assign((root_index >> 5) + 2, 0u);
             for (size_t i = 0; i < deep.size(); i++) {
                 if (in_hot[i]) continue;
                 const uint32_t hh = deep[i].key * 0x9E3779B1u;
-                uint32_t slot = (hh ^ (hh >> 15)) & cold_mask;
-                while (cold[slot].x != T_EMPTY_KEY) slot = (slot + 1) & cold_mask;
+                size_t slot = (size_t)((hh ^ (hh >> 15)) & cold_mask) * 2;
+                while (cold[slot].x != T_EMPTY_KEY) slot = (slot + 1) & (cold.size() - 1);
                 cold[slot] = make_uint2(deep[i].key, deep[i].value);
                 cold_bits[deep[i].parent >> 5] |= 1u << (deep[i].parent & 31u);
             }
