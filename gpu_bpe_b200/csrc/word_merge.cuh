@@ -12,7 +12,7 @@
 // counts), and the barriers between its two phases, not bandwidth.  So the loop runs inside ONE thread-block cluster: 16 CTAs on
 // 16 SMs, whose hardware barrier costs a fraction of a grid-wide one, with the arg-max exchanged through distributed shared
 // memory.  Against full passes over the symbol buffers (train_kernels.cuh, which "literal" compaction and sharded runs take): 64 MiB,
-// 8,000 merges 522 -> 85 ms; heavy-tailed 256 MiB, 4,000 merges 1,326 -> 77 ms; 1 GiB, 32,000 merges 16.5 -> 0.46 s.
+// 8,000 merges 522 -> 64 ms; heavy-tailed 256 MiB, 4,000 merges 1,326 -> 70 ms.
 // Phase 1 finds and verifies the occurrences (all reads see the state before the merge), updates the pair table and
 // writes the list of the new symbol; phase 2 rewrites the records and takes the arg-max of the next merge.
 #pragma once
@@ -26,7 +26,7 @@ namespace b200bpe {
 constexpr int WM_THREADS = 512;
 constexpr int WM_CLUSTER = 16;             // CTAs (the largest cluster the hardware takes)
 constexpr int WM_QUEUE = 6144;             // occurrences a CTA keeps in shared memory between the phases
-constexpr int WM_UNROLL = 4;               // list entries a thread has in flight
+constexpr int WM_UNROLL = 8;               // list entries a thread has in flight
 constexpr int WM_CAND = 2048;              // candidates per CTA
 constexpr uint32_t WM_CAND_GOAL = 6000;    // candidates a scan aims at, all CTAs together
 constexpr int WM_BINS = 256;
@@ -57,6 +57,8 @@ struct WordArgs {
     const uint32_t* byte_off;
     uint2* entries;                   // {position of the left symbol, left << 16 | right}
     uint2* segment;                   // [symbol] = {first entry, end}
+    uint32_t* usual;                  // [symbol] = positions it usually covers (always, but for symbols made of a run of equal ones)
+    uint32_t positions;               // rec[positions] begins a word, and nothing lies behind it
     unsigned long long* table;        // pair << 32 | count, pair = left << 16 | right, never 0
     uint32_t table_log2;
     uint32_t* cand;                   // candidates between launches: [WM_CLUSTER][WM_CAND + 1], count first
@@ -152,39 +154,71 @@ struct WordTeam {
     cooperative_groups::cluster_group cluster;
 };
 
-// Count update of one pair.  `tau` as in WordState; a rise across it makes the slot a candidate of this CTA.
-__device__ __forceinline__ void wt_update(const WordArgs& A, WordTeam& T, uint32_t pair, uint32_t slot, unsigned long long seen, uint32_t w, bool rise,
-                                          unsigned long long tau) {
-    const uint32_t mask = (1u << A.table_log2) - 1u;
-    for (int p = 0; p < WM_MAX_PROBE; p++) {
-        if (seen == 0ull) {
-            if (!rise) break;       // a pair that occurs is in the table
-            const unsigned long long fresh = (unsigned long long)pair << 32 | w;
-            seen = atomicCAS(A.table + slot, 0ull, fresh);
-            if (seen == 0ull) {
-                atomicAdd(&T.s.inserted, 1u);
-                if (wt_rank(fresh) >= tau) {
-                    const uint32_t i = atomicAdd(&T.s.ncand, 1u);
-                    if (i < WM_CAND) T.s.cand[i] = slot; else atomicOr(&T.s.flags, (uint32_t)WS_CAND);
-                }
-                return;
-            }
-        }
-        if ((uint32_t)(seen >> 32) == pair) {
-            uint32_t* count = reinterpret_cast<uint32_t*>(A.table + slot);   // the lower half
-            if (!rise) { atomicSub(count, w); return; }
-            const uint32_t old = atomicAdd(count, w);
-            const unsigned long long low = (uint32_t)~pair;
-            if (((unsigned long long)old << 32 | low) < tau && ((unsigned long long)(old + w) << 32 | low) >= tau) {
-                const uint32_t i = atomicAdd(&T.s.ncand, 1u);
-                if (i < WM_CAND) T.s.cand[i] = slot; else atomicOr(&T.s.flags, (uint32_t)WS_CAND);
-            }
-            return;
-        }
-        slot = (slot + 1u) & mask;
-        seen = __ldcg(A.table + slot);
+// Count updates of up to N pairs by one thread, in step: their probes, insertions and adds are in flight together.  One after the other they
+// were 6,000 of the 10,000 cycles of phase 1, and most of the wait at the barrier behind it: 64 MiB, 8,000 merges 85 -> 65 ms.  wanted: bit k = pair[k] changes by w[k]; rise: bit k = upwards.  `tau` as in
+// WordState; a rise across it makes the slot a candidate of this CTA.
+template <int N>
+__device__ __forceinline__ void wt_updates(const WordArgs& A, WordTeam& T, const uint32_t (&pair)[N], const uint32_t (&w)[N], uint32_t wanted, uint32_t rise,
+                                           unsigned long long tau) {
+    const uint32_t mask = (1u << A.table_log2) - 1u, sh = 32u - A.table_log2;
+    uint32_t slot[N];
+    unsigned long long seen[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        slot[k] = wt_hash(pair[k]) >> sh;
+        seen[k] = (wanted >> k) & 1u ? __ldcg(A.table + slot[k]) : 0ull;
     }
-    atomicOr(&T.s.flags, (uint32_t)WS_FULL);
+    auto candidate = [&](uint32_t at) {
+        const uint32_t i = atomicAdd(&T.s.ncand, 1u);
+        if (i < WM_CAND) T.s.cand[i] = at; else atomicOr(&T.s.flags, (uint32_t)WS_CAND);
+    };
+    uint32_t open = wanted, found = 0u;
+    for (int p = 0; open && p < WM_MAX_PROBE; p++) {
+        uint32_t tried = 0u;
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            if (((open >> k) & 1u) && seen[k] == 0ull) {
+                if ((rise >> k) & 1u) { seen[k] = atomicCAS(A.table + slot[k], 0ull, (unsigned long long)pair[k] << 32 | w[k]); tried |= 1u << k; }
+                else { atomicOr(&T.s.flags, (uint32_t)WS_FULL); open &= ~(1u << k); }       // a pair that occurs is in the table
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            if (!((open >> k) & 1u)) continue;
+            if (((tried >> k) & 1u) && seen[k] == 0ull) {                                   // inserted
+                open &= ~(1u << k);
+                atomicAdd(&T.s.inserted, 1u);
+                if (wt_rank((unsigned long long)pair[k] << 32 | w[k]) >= tau) candidate(slot[k]);
+            } else if ((uint32_t)(seen[k] >> 32) == pair[k]) {
+                open &= ~(1u << k);
+                found |= 1u << k;
+            } else {
+                slot[k] = (slot[k] + 1u) & mask;
+                seen[k] = __ldcg(A.table + slot[k]);
+            }
+        }
+    }
+    if (open) atomicOr(&T.s.flags, (uint32_t)WS_FULL);
+    int old[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        old[k] = 0;
+        if (!((found >> k) & 1u)) continue;
+        uint32_t* count = reinterpret_cast<uint32_t*>(A.table + slot[k]);   // the lower half
+        if ((rise >> k) & 1u) old[k] = (int)atomicAdd(count, w[k]); else atomicSub(count, w[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        if (!((found & rise) >> k & 1u)) continue;
+        // (in a "literal" run the rises and falls of a merge come in any order, so that a count can be below 0 on the way)
+        const int now = old[k] + (int)w[k];
+        const unsigned long long low = (uint32_t)~pair[k];
+        if (now > 0 && ((unsigned long long)max(old[k], 0) << 32 | low) < tau && ((unsigned long long)now << 32 | low) >= tau) candidate(slot[k]);
+    }
+}
+__device__ __forceinline__ void wt_update(const WordArgs& A, WordTeam& T, uint32_t pair, uint32_t w, bool rise, unsigned long long tau) {
+    const uint32_t k[1] = {pair}, v[1] = {w};
+    wt_updates<1>(A, T, k, v, 1u, rise ? 1u : 0u, tau);
 }
 
 // Best candidate of the cluster and the CTAs' flags; ends with the cluster barrier that also publishes phase 2's writes.
@@ -345,6 +379,7 @@ k_word_merges(WordArgs A, uint32_t target) {
         if (bytes) { beg = __ldcg(A.byte_off + (a << 8 | b)); end = __ldcg(A.byte_off + (a << 8 | b) + 1); }
         else { const uint2 g = __ldcg(A.segment + max(a, b)); beg = g.x; end = g.y; }
         const uint32_t len = end - beg;
+        const uint32_t usual_a = a < 256u ? 1u : __ldcg(A.usual + a), usual_b = b < 256u ? 1u : __ldcg(A.usual + b);
         // a merge makes at most two new pairs per symbol in use, and per occurrence
         const uint32_t grow = 2u * min(min(len, count), fresh + 1u);
         if (occ_most + grow > room) {
@@ -356,17 +391,21 @@ k_word_merges(WordArgs A, uint32_t target) {
         // ── phase 1: occurrences, counts, the new symbol's list ──
         auto apply = [&](uint32_t qi) {
             const uint32_t p = s.queue[qi].x;
-            const uint32_t rp = A.rec[p], w = A.weight[p];
-            const uint32_t prev_end = (rp & WP_START) ? 0u : A.rec[p - 1];
+            // every record that is usually needed, in one round trip: the second symbol and the one behind it where they usually are
+            // (64 MiB, 8,000 merges: 65.4 -> 63.9 ms)
+            const uint32_t q_usual = min(p + usual_a, A.positions), r_usual = min(p + usual_a + usual_b, A.positions);
+            const uint32_t rp = A.rec[p], w = A.weight[p], rec_before = p > 0u ? A.rec[p - 1] : 0u;
+            const uint32_t rec_q = A.rec[q_usual], rec_r = A.rec[r_usual];
+            const uint32_t prev_end = (rp & WP_START) ? 0u : rec_before;
             bool ok = wp_sym(rp) == a;
             const uint32_t la = wp_span(rp), q = p + la;
-            const uint32_t rq = ok ? A.rec[q] : WP_START;
+            const uint32_t rq = !ok ? WP_START : q == q_usual ? rec_q : A.rec[q];
             ok = ok && !(rq & WP_START) && wp_sym(rq) == b;
             // the left neighbour: symbol x at l
             uint32_t l = 0u, x = 0u, rl = WP_START;
             if (ok && !(rp & WP_START)) { l = p - wp_span(prev_end); rl = A.rec[l]; x = wp_sym(rl); }
             if (a == b && x == a) ok = false;         // inside a run of equal symbols: its first position merges the whole run
-            uint32_t r = q + wp_span(rq), rr = ok ? A.rec[r] : WP_START;
+            uint32_t r = q + wp_span(rq), rr = !ok ? WP_START : r == r_usual ? rec_r : A.rec[r];
             if (a == b) while (ok && !(rr & WP_START) && wp_sym(rr) == a) { r += wp_span(rr); rr = A.rec[r]; }
             const uint32_t span = r - p;
             uint32_t y = (!ok || (rr & WP_START)) ? 0u : wp_sym(rr);
@@ -386,38 +425,21 @@ k_word_merges(WordArgs A, uint32_t target) {
             }
             const bool right = y != 0u;
             s.queue[qi] = ok ? make_uint2(p, span | (a == b ? 0u : la << 16)) : make_uint2(~0u, 0u);
-            // room in the list of the new symbol
+            // the four counts that change
+            const uint32_t k0 = x << 16 | a, k1 = x << 16 | fresh, k2 = right_left << 16 | y, k3 = fresh << 16 | new_right;
+            // room in the list of the new symbol: asked for now, needed last (the counter is in another SM)
             const uint32_t want = (left ? 1u : 0u) + (right ? 1u : 0u);
             const uint32_t active = __activemask();
+            const uint32_t one = __ballot_sync(active, want & 1u), two = __ballot_sync(active, want & 2u);
+            const int leader = __ffs((int)active) - 1;
             uint32_t at = 0u;
-            {
-                const uint32_t one = __ballot_sync(active, want & 1u), two = __ballot_sync(active, want & 2u);
-                const uint32_t total = __popc(one) + 2u * __popc(two);
-                if (total) {
-                    const int leader = __ffs((int)active) - 1;
-                    if ((int)lane == leader) at = atomicAdd(&T.lead->c_entries, total);
-                    at = __shfl_sync(active, at, leader);
-                    const uint32_t below = (1u << lane) - 1u;
-                    at += __popc(one & below) + 2u * __popc(two & below);
-                }
-            }
-            // the four counts that change; all first probes in flight together
-            const uint32_t k0 = x << 16 | a, k1 = x << 16 | fresh, k2 = right_left << 16 | y, k3 = fresh << 16 | new_right;
-            const uint32_t sh = 32u - A.table_log2;
-            const uint32_t s0 = wt_hash(k0) >> sh, s1 = wt_hash(k1) >> sh, s2 = wt_hash(k2) >> sh, s3 = wt_hash(k3) >> sh;
-            unsigned long long v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-            if (left) { v0 = __ldcg(A.table + s0); v1 = __ldcg(A.table + s1); }
-            if (right) { v2 = __ldcg(A.table + s2); v3 = __ldcg(A.table + s3); }
-            if (left) {
-                A.entries[at++] = make_uint2(l, k1);
-                wt_update(A, T, k0, s0, v0, w, false, tau);
-                wt_update(A, T, k1, s1, v1, w, true, tau);
-            }
-            if (right) {
-                A.entries[at] = make_uint2(p, k3);
-                wt_update(A, T, k2, s2, v2, w, false, tau);
-                wt_update(A, T, k3, s3, v3, w, true, tau);
-            }
+            if ((int)lane == leader && (one | two)) at = atomicAdd(&T.lead->c_entries, __popc(one) + 2u * __popc(two));
+            const uint32_t keys[4] = {k0, k1, k2, k3}, by[4] = {w, w, w, w};
+            wt_updates<4>(A, T, keys, by, (left ? 3u : 0u) | (right ? 12u : 0u), 10u, tau);
+            const uint32_t below = (1u << lane) - 1u;
+            at = __shfl_sync(active, at, leader) + __popc(one & below) + 2u * __popc(two & below);
+            if (left) A.entries[at++] = make_uint2(l, k1);
+            if (right) A.entries[at] = make_uint2(p, k3);
         };
         // Phase 2 of one occurrence.
         auto rewrite = [&](uint32_t qi) {
@@ -485,8 +507,7 @@ k_word_merges(WordArgs A, uint32_t target) {
         const bool spilled = walk(apply);
         if (gtid == 0) {
             // every occurrence of the pair itself goes
-            const uint32_t sl = wt_hash(pair) >> (32u - A.table_log2);
-            wt_update(A, T, pair, sl, __ldcg(A.table + sl), count, false, tau);
+            wt_update(A, T, pair, count, false, tau);
         }
         __syncwarp();
         cluster_barrier();
@@ -521,6 +542,7 @@ k_word_merges(WordArgs A, uint32_t target) {
         if (gtid == 0) {
             const uint32_t e1 = s.c_entries;
             A.segment[fresh] = make_uint2(s.init.entries, e1);
+            A.usual[fresh] = usual_a + usual_b;
             s.init.entries = e1;
             A.log[done] = make_uint4(a, b, fresh, count);
         }

@@ -40,7 +40,7 @@ struct WordPath {
         if (!ctx) return;
         for (void* p : {(void*)dict.short_key, (void*)dict.short_cnt, (void*)dict.short_base, (void*)dict.long_key, (void*)dict.long_cnt,
                         (void*)dict.long_base, (void*)dict.st, (void*)args.rec, (void*)args.weight, (void*)args.byte_list, (void*)args.byte_off,
-                        (void*)args.entries, (void*)args.segment, (void*)args.table, (void*)args.cand, (void*)args.st, (void*)args.log,
+                        (void*)args.entries, (void*)args.segment, (void*)args.usual, (void*)args.table, (void*)args.cand, (void*)args.st, (void*)args.log,
                         (void*)cursor, (void*)bins, (void*)own_mask, (void*)own_bytes})
             ctx->free(p);
         if (h_state) cudaFreeHost(h_state);
@@ -70,6 +70,7 @@ struct WordPath {
         B2_CUDA(ctx->alloc(&cursor, sizeof(uint32_t) * 65536));
         B2_CUDA(ctx->alloc(&bins, sizeof(unsigned long long) * 65536));
         B2_CUDA(ctx->alloc(&args.segment, sizeof(uint2) * 65536));
+        B2_CUDA(ctx->alloc(&args.usual, sizeof(uint32_t) * 65536));
         B2_CUDA(ctx->alloc(&args.cand, sizeof(uint32_t) * WM_CLUSTER * (WM_CAND + 1)));
         B2_CUDA(ctx->alloc(&args.st, sizeof(WordState)));
         B2_CUDA(ctx->alloc(&args.log, sizeof(uint4) * (size_t)goal));
@@ -127,6 +128,7 @@ struct WordPath {
         B2_CUDA(cudaGetLastError());
         if (h_dict->status) return B200BPE_OK;
         positions = h_dict->positions;
+        args.positions = positions;
         if (positions > cap_positions || !args.rec) {
             for (void* p : {(void*)args.rec, (void*)args.weight, (void*)args.byte_list, (void*)args.entries}) ctx->free(p);
             args.rec = nullptr; args.weight = nullptr; args.byte_list = nullptr; args.entries = nullptr;
@@ -146,10 +148,11 @@ struct WordPath {
         k_dict_offsets<<<1, 1024, 0, s>>>(bins, off, cursor, dict.st);
         k_dict_lists<<<blocks(positions, 256, 8), 256, 0, s>>>(args.rec, positions, cursor, list);
         launches += 4;
-        // The table has room for twice the byte pairs there can be at most; it grows when merges fill it.
+        // The table has room for twice the byte pairs there can be at most; it grows when merges fill it.  It is sparse (two slots a position
+        // at most): a probe that collides is another round trip, and the scans that pay for its size are a few in a run.
         if (args.table_log2 == 0) {
             uint32_t l = 13;
-            while (l < 22 && (8ull << l) < positions) l++;
+            while (l < 23 && (2ull << l) < positions) l++;
             args.table_log2 = l;
         }
         uint64_t most = std::min<uint64_t>(positions, 65536);
