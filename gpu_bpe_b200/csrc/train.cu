@@ -279,10 +279,10 @@ b200bpe_status Trainer::alloc_common() {
     return B200BPE_OK;
 }
 
-// Which runs train on the dictionary of distinct words: "fixed" compaction on one GPU, new ids above the byte values, no option that
+// Which runs train on the dictionary of distinct words: those on one GPU, new ids above the byte values, no option that
 // is about the other path's kernels (a recount per merge, the test of its bounded wait).  Positions are 32-bit with a bit to spare.
 bool Trainer::words_eligible() const {
-    return ctx->world == 1 && opts.compat_mode == B200BPE_COMPAT_FIXED && !(opts.flags & B200BPE_FLAG_FULL_RECOUNT) && !opts.test_first_tile &&
+    return ctx->world == 1 && !(opts.flags & B200BPE_FLAG_FULL_RECOUNT) && !opts.test_first_tile &&
            opts.first_token_id >= 256 && n0 < (1ull << 31);
 }
 
@@ -300,7 +300,7 @@ b200bpe_status Trainer::init_state() {
     if (words_eligible()) {
         if (!words) {
             words = new WordPath();
-            b200bpe_status r = words->create(ctx, n0, merges_goal, opts.table_log2);
+            b200bpe_status r = words->create(ctx, n0, merges_goal, opts.table_log2, opts.compat_mode == B200BPE_COMPAT_LITERAL);
             if (r) return r;
         }
         const uint64_t before = words->launches;
@@ -555,11 +555,20 @@ b200bpe_status Trainer::run_words(uint32_t until, uint32_t start_done, uint32_t*
         const WordState st = w.h_state[i];
         tail++;
         if (st.status & ~(uint32_t)WS_GROW) {
-            // a pair table or candidate list that filled up within one merge: run again on the symbol buffers
             B2_CUDA(cudaStreamSynchronize(s));
             by_words = false;
             early_stop = false;
             const uint32_t had = merges_done;
+            if (st.status == WS_TAIL && had == 0 && w.tail_share < WordPath::TAIL_LONG) {
+                // a "literal" run whose tail is too short for its first merges: the same again with a longer one
+                w.tail_share = WordPath::TAIL_LONG;
+                const uint64_t before = w.launches;
+                b200bpe_status r = w.build(d_bytes, has_mask ? d_mask : nullptr, d_sym_init, opts.first_token_id, &by_words);
+                if (r) return r;
+                launches += w.launches - before;
+                if (by_words) { head = tail = 0; enqueued = 0; continue; }
+            }
+            // a pair table or candidate list that filled up within one merge: run again on the symbol buffers
             merges_done = 0;
             cur_n = n0;
             b200bpe_status r = init_classic();
@@ -578,6 +587,7 @@ b200bpe_status Trainer::run_words(uint32_t until, uint32_t start_done, uint32_t*
             if (merges_out) { merges_out[o * 3 + 0] = l.x; merges_out[o * 3 + 1] = l.y; merges_out[o * 3 + 2] = l.z; }
             if (counts_out) counts_out[o] = l.w;
         }
+        w.seen = st;
         const bool got = st.merges_done != merges_done;
         merges_done = st.merges_done;
         cur_n = st.symbols;

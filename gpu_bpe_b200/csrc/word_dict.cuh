@@ -32,6 +32,7 @@ struct DictState {
     uint32_t positions;      // symbols of all distinct words
     uint32_t words;          // distinct words
     uint32_t pairs;          // distinct byte pairs
+    unsigned long long split;   // "literal" runs: where the tail begins
 };
 
 struct DictTables {
@@ -446,6 +447,34 @@ k_dict_split(const uint32_t* __restrict__ sym, uint64_t n, uint8_t* __restrict__
         mask[i] = (s & WORD_START_BIT) ? 1 : 0;
     }
     if (bad) atomicOr(&st->status, (uint32_t)WD_SYMBOL);
+}
+
+// ── the tail of a "literal" run ──
+// First word start at or behind `from`, or n (one CTA; a text without one within WD_MAX_WORD bytes is not one of words).
+__global__ void __launch_bounds__(256)
+k_dict_split_at(const uint8_t* __restrict__ mask, uint64_t n, uint64_t from, DictState* __restrict__ st) {
+    for (uint64_t b = from; b < n && b <= from + WD_MAX_WORD; b += 256) {
+        __shared__ uint32_t best;
+        if (threadIdx.x == 0) best = 256u;
+        __syncthreads();
+        if (b + threadIdx.x < n && mask[b + threadIdx.x]) atomicMin(&best, threadIdx.x);
+        __syncthreads();
+        if (best < 256u) { if (threadIdx.x == 0) st->split = b + best; return; }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) st->split = n;
+}
+// Tagged symbols of the tail, and its byte pairs in the lower halves of the bins.
+__global__ void __launch_bounds__(256)
+k_dict_tail(const uint8_t* __restrict__ bytes, const uint8_t* __restrict__ mask, uint64_t at, uint64_t n, uint32_t* __restrict__ tail,
+            unsigned long long* __restrict__ bins) {
+    for (uint64_t i = at + (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256) {
+        const uint32_t l = bytes[i];
+        tail[i - at] = l | (mask[i] ? WORD_START_BIT : 0u);
+        if (i + 1 >= n || mask[i + 1]) continue;
+        const uint32_t r = bytes[i + 1];
+        if (l && r) atomicAdd(bins + (l << 8 | r), 1ull);
+    }
 }
 
 // ── the live symbols, in text order ──

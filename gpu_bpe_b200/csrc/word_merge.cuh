@@ -11,7 +11,7 @@
 // What bounds a merge is then a chain of dependent memory round trips (occurrence list -> records -> pair table -> candidates'
 // counts), and the barriers between its two phases, not bandwidth.  So the loop runs inside ONE thread-block cluster: 16 CTAs on
 // 16 SMs, whose hardware barrier costs a fraction of a grid-wide one, with the arg-max exchanged through distributed shared
-// memory.  Against full passes over the symbol buffers (train_kernels.cuh, which "literal" compaction and sharded runs take): 64 MiB,
+// memory.  Against full passes over the symbol buffers (train_kernels.cuh, which sharded runs take): 64 MiB,
 // 8,000 merges 522 -> 64 ms; heavy-tailed 256 MiB, 4,000 merges 1,326 -> 70 ms.
 // Phase 1 finds and verifies the occurrences (all reads see the state before the merge), updates the pair table and
 // writes the list of the new symbol; phase 2 rewrites the records and takes the arg-max of the next merge.
@@ -33,7 +33,7 @@ constexpr int WM_BINS = 256;
 constexpr int WM_MAX_PROBE = 4096;
 
 // Why the loop stopped (WordState::status).
-enum : uint32_t { WS_OK = 0, WS_GROW = 1u, WS_FULL = 2u, WS_CAND = 4u };
+enum : uint32_t { WS_OK = 0, WS_GROW = 1u, WS_FULL = 2u, WS_CAND = 4u, WS_TAIL = 8u };
 
 struct __align__(16) WordState {
     unsigned long long tau;      // threshold of the candidate list, as count << 32 | ~pair; ~0 = no list
@@ -47,7 +47,8 @@ struct __align__(16) WordState {
     uint32_t occupied;           // pair table slots in use
     uint32_t symbols;            // live symbols of the corpus
     uint32_t scans;              // table scans so far (statistics)
-    uint32_t pad[3];
+    uint32_t front, front_before;   // "literal" runs: symbols of the dictionary's part, now and before the last merge
+    uint32_t turn;               // and merges so far, which say which tail buffer is which
 };
 
 struct WordArgs {
@@ -62,6 +63,7 @@ struct WordArgs {
     unsigned long long* table;        // pair << 32 | count, pair = left << 16 | right, never 0
     uint32_t table_log2;
     uint32_t* cand;                   // candidates between launches: [WM_CLUSTER][WM_CAND + 1], count first
+    uint32_t* tail[3];                // "literal" runs: the symbols behind the dictionary's words
     WordState* st;
     uint4* log;                       // {a, b, new_id, count} per merge
 };
@@ -74,7 +76,9 @@ struct WordShared {
     uint32_t xflags[WM_CLUSTER];
     unsigned long long wbest[WM_THREADS / 32];
     uint32_t queued, ncand, flags, inserted;
-    uint32_t c_entries, c_inserted;   // the cluster's counters: those of CTA 0 are the ones in use
+    uint32_t c_entries, c_inserted, c_merged;   // the cluster's counters: those of CTA 0 are the ones in use
+    uint32_t xkept[WM_CLUSTER], wkept[WM_THREADS / 32];   // tail symbols that a CTA, a warp copies
+    uint32_t tail_queue[4096], tail_queued;               // matches in this CTA's part of the tail
     WordState init;
 };
 
@@ -110,7 +114,7 @@ __device__ __forceinline__ bool wt_insert(unsigned long long* __restrict__ table
 // The byte pairs of the corpus, and the control block of a fresh run.
 __global__ void __launch_bounds__(256)
 k_word_init(const unsigned long long* __restrict__ bins, const DictState* __restrict__ ds, unsigned long long* __restrict__ table, uint32_t log2,
-            WordState* __restrict__ st, uint32_t first_id, uint32_t n) {
+            WordState* __restrict__ st, uint32_t first_id, uint32_t n, uint32_t front) {
     const uint32_t i = blockIdx.x * 256 + threadIdx.x;      // 65,536 threads
     const unsigned long long v = bins[i];
     const uint32_t pair = (i >> 8) << 16 | (i & 0xFFu);
@@ -119,6 +123,7 @@ k_word_init(const unsigned long long* __restrict__ bins, const DictState* __rest
         st->tau = ~0ull;
         st->next_id = first_id;
         st->symbols = n;
+        st->front = st->front_before = front;
         st->occupied = ds->pairs;
     }
 }
@@ -331,6 +336,222 @@ __device__ __noinline__ void word_scan(const WordArgs& A, WordTeam& T, unsigned 
     __syncthreads();
 }
 
+// ── the tail of a "literal" run ──
+// "literal" compaction bounds its INPUT by the post-merge count (train.wgsl:698,727), so a merge of count c drops the last c symbols and
+// leaves as many positions to what the destination held two merges ago.  Everything this ever touches lies near the end of the text:
+// the dictionary takes the words of its front, where a merge does what it does in "fixed" mode, and the symbols behind them are kept one
+// by one, in three buffers that take turns (this merge's source, the one before it, the destination).  `symbols` counts both parts; the
+// tail's first symbol begins a word and is never dropped.  A merge that reaches past the tail ends the run here (WS_TAIL): the symbol
+// buffers then take it from its start.
+//
+// A merge reads the tail twice: phase 1 counts what every warp's share keeps and updates the pairs that change; phase 2, with every
+// offset known, writes the destination, rewrites the source in place as the reference does (train.wgsl:486-487: the next merge but one may see it),
+// and copies the older symbols in.  The pairs' counts can rise here at any time, unlike the dictionary's.
+struct TailView {
+    const uint32_t* cur;
+    uint32_t n, limit;           // its symbols; the first `limit` are copied
+    uint32_t a, b, fresh;
+};
+__device__ __forceinline__ bool tail_counted(uint32_t l, uint32_t r) { return !(r & WORD_START_BIT) && (l & TOKEN_MASK) && (r & TOKEN_MASK); }
+// A source symbol as it was before this merge (the new id does not occur otherwise).
+__device__ __forceinline__ uint32_t tail_before(const TailView& v, uint32_t s) { return (s & TOKEN_MASK) == v.fresh ? (s & WORD_START_BIT) | v.a : s; }
+__device__ __forceinline__ bool tail_match(const TailView& v, uint32_t l, uint32_t r) {
+    return (l & TOKEN_MASK) == v.a && (r & (TOKEN_MASK | WORD_START_BIT)) == v.b;
+}
+__device__ __forceinline__ uint32_t tail_at(const TailView& v, uint32_t i) {      // beyond the end: a word start, which ends everything
+    return i < v.n ? tail_before(v, __ldcg(v.cur + i)) : WORD_START_BIT;
+}
+__device__ __forceinline__ void tail_pair(const WordArgs& A, WordTeam& T, uint32_t l, uint32_t r, bool rise, unsigned long long tau) {
+    const uint32_t pair = (l & TOKEN_MASK) << 16 | (r & TOKEN_MASK);
+    wt_update(A, T, pair, 1u, rise, tau);
+}
+// The changes at position i < limit: the pair that begins there goes unless it is copied as it is (from limit - 1 on all pairs go: tail_pairs);
+// what the symbol there is copied next to comes.
+__device__ __forceinline__ void tail_changes(const WordArgs& A, WordTeam& T, const TailView& v, uint32_t i, unsigned long long tau) {
+    const uint32_t sm = i > 0u ? tail_at(v, i - 1u) : WORD_START_BIT, s0 = tail_at(v, i), s1 = tail_at(v, i + 1u), s2 = tail_at(v, i + 2u);
+    const bool ml = i > 0u && tail_match(v, sm, s0), mi = tail_match(v, s0, s1), mr = tail_match(v, s1, s2);
+    if (tail_counted(s0, s1) && i + 1u < v.limit && (ml || mi || mr)) tail_pair(A, T, s0, s1, false, tau);
+    if (ml) return;
+    uint32_t j = i + 1u, before = s0, s = s1;
+    while (tail_match(v, before, s)) { before = s; s = tail_at(v, ++j); }
+    if (j >= v.limit) return;              // (what the last copied symbol ends up next to is known in phase 2)
+    const bool mj = tail_match(v, s, tail_at(v, j + 1u));
+    if (!(mi || mj)) return;
+    const uint32_t l = mi ? v.fresh : s0, r = mj ? (s & WORD_START_BIT) | v.fresh : s;
+    if (tail_counted(l, r)) tail_pair(A, T, l, r, true, tau);
+}
+// The same for all positions around a match at m < limit that no earlier match sees to, with everything in flight together.
+__device__ __forceinline__ void tail_match_changes(const WordArgs& A, WordTeam& T, const TailView& v, uint32_t m, unsigned long long tau) {
+    uint32_t t[7];          // symbols m - 2 .. m + 4
+#pragma unroll
+    for (int k = 0; k < 7; k++) t[k] = m + k >= 2u ? tail_at(v, m + k - 2u) : WORD_START_BIT;
+    const bool m2 = m >= 2u && tail_match(v, t[0], t[1]), m1 = m >= 1u && tail_match(v, t[1], t[2]);     // at m - 2, m - 1
+    const bool n1 = tail_match(v, t[3], t[4]), n2 = tail_match(v, t[4], t[5]);                            // at m + 1, m + 2
+    if (v.a == v.b) {       // runs of any length
+        tail_changes(A, T, v, m, tau);
+        if (!n1) { if (m + 1u < v.limit) tail_changes(A, T, v, m + 1u, tau); }
+        if (m >= 1u && !m1 && !m2) tail_changes(A, T, v, m - 1u, tau);
+        return;
+    }
+    // (a != b: a match is never next to another one; m + 2 may be the next)
+    const bool before = m >= 1u && !m2;                     // position m - 1 is this match's to see to
+    uint32_t pair[5], wanted = 0u;
+    const uint32_t one[5] = {1u, 1u, 1u, 1u, 1u};
+    auto put = [&](int k, uint32_t l, uint32_t r, bool yes) {
+        pair[k] = (l & TOKEN_MASK) << 16 | (r & TOKEN_MASK);
+        if (yes && tail_counted(l, r)) wanted |= 1u << k;
+    };
+    put(0, t[1], t[2], before && m < v.limit);              // falls
+    put(1, t[2], t[3], m + 1u < v.limit);
+    put(2, t[3], t[4], m + 2u < v.limit);
+    put(3, t[1], (t[2] & WORD_START_BIT) | v.fresh, before);                                             // rises
+    put(4, v.fresh, n2 ? (t[4] & WORD_START_BIT) | v.fresh : t[4], m + 2u < v.limit);
+    wt_updates<5>(A, T, pair, one, wanted, 24u, tau);
+}
+// The tail goes by in spans of TAIL_SPAN symbols: four 16-byte loads per lane.  match: bit 4 u + k = a pair begins at symbol k of the lane's
+// u-th four; left: one begins right before the span.
+constexpr uint32_t TAIL_SPAN = 512;
+constexpr uint32_t TAIL_QUEUE = 4096;
+struct TailSpan { uint4 q[4]; uint32_t match; bool left; };
+__device__ __forceinline__ void tail_span(const TailView& v, uint32_t base, uint32_t lane, TailSpan& t) {
+    if (base + TAIL_SPAN <= v.limit) {          // (behind the limit the rewrite is under way in phase 2)
+        const uint4* __restrict__ p = reinterpret_cast<const uint4*>(v.cur + base) + lane;
+#pragma unroll
+        for (int u = 0; u < 4; u++) t.q[u] = __ldcg(p + u * 32);
+    } else {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t i = base + u * 128u + lane * 4u;
+            t.q[u] = make_uint4(tail_at(v, i), tail_at(v, i + 1u), tail_at(v, i + 2u), tail_at(v, i + 3u));
+        }
+    }
+    uint32_t edge = 0u;
+    if (lane < 2u) edge = lane == 0u ? (base > 0u ? tail_at(v, base - 1u) : WORD_START_BIT) : tail_at(v, base + TAIL_SPAN);
+    const uint32_t before = __shfl_sync(0xFFFFFFFFu, edge, 0), behind = __shfl_sync(0xFFFFFFFFu, edge, 1);
+    t.match = 0u;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        uint32_t nx = __shfl_down_sync(0xFFFFFFFFu, t.q[u].x, 1);
+        const uint32_t far = u < 3 ? __shfl_sync(0xFFFFFFFFu, t.q[u < 3 ? u + 1 : u].x, 0) : behind;
+        if (lane == 31) nx = far;
+        t.match |= (tail_match(v, t.q[u].x, t.q[u].y) ? 1u : 0u) << (4 * u) | (tail_match(v, t.q[u].y, t.q[u].z) ? 2u : 0u) << (4 * u) |
+                   (tail_match(v, t.q[u].z, t.q[u].w) ? 4u : 0u) << (4 * u) | (tail_match(v, t.q[u].w, nx) ? 8u : 0u) << (4 * u);
+    }
+    t.left = tail_match(v, before, __shfl_sync(0xFFFFFFFFu, t.q[0].x, 0));
+}
+// Phase 1 over [from, to), whole spans but for the last: queues the matches, and returns how many symbols are copied (the same in every lane).
+__device__ __forceinline__ uint32_t tail_count(const WordArgs& A, WordTeam& T, const TailView& v, uint32_t from, uint32_t to, unsigned long long tau) {
+    const uint32_t lane = T.tid & 31;
+    uint32_t kept = to - from;
+    for (uint32_t span = from; span < to; span += TAIL_SPAN) {
+        TailSpan t;
+        tail_span(v, span, lane, t);
+        const uint32_t end = to - span;           // symbols of the span that are in question
+        uint32_t match = t.match, drops = 0u;
+        if (end < TAIL_SPAN) {
+#pragma unroll
+            for (int k = 0; k < 16; k++) if ((uint32_t)(k / 4) * 128u + lane * 4u + k % 4 >= end) match &= ~(1u << k);
+        }
+        if (__any_sync(0xFFFFFFFFu, match != 0u)) {
+            // what a match drops is the symbol behind it, if that is still in question
+            const uint32_t last = span + TAIL_SPAN < to ? TAIL_SPAN : end;
+            drops = __popc(match);
+            const uint32_t at_end = last - 1u;    // (the position whose successor belongs to the next span or warp)
+            if (at_end % 128u / 4u == lane && ((match >> (at_end / 128u * 4u + at_end % 4u)) & 1u)) drops--;
+            drops = __reduce_add_sync(0xFFFFFFFFu, drops);
+            while (match) {
+                const uint32_t k = (uint32_t)__ffs((int)match) - 1u, m = span + k / 4u * 128u + lane * 4u + k % 4u;
+                match &= match - 1u;
+                const uint32_t i = atomicAdd(&T.s.tail_queued, 1u);
+                if (i < TAIL_QUEUE) T.s.tail_queue[i] = m; else tail_match_changes(A, T, v, m, tau);
+            }
+            __syncwarp();
+        }
+        kept -= drops + (t.left ? 1u : 0u);
+    }
+    return kept;
+}
+// Pairs of neighbours among `n` symbols at s (with the one behind them): all of them go, or come; several in flight per thread.
+__device__ __forceinline__ void tail_pairs(const WordArgs& A, WordTeam& T, const uint32_t* __restrict__ s, uint32_t n, uint32_t first, bool rise,
+                                           unsigned long long tau, uint32_t* __restrict__ copy) {
+    constexpr int U = 4;
+    constexpr uint32_t STEP = WM_THREADS * WM_CLUSTER;
+    for (uint32_t i0 = first; i0 < n; i0 += STEP * U) {
+        uint32_t l[U], r[U], pair[U], wanted = 0u;
+        const uint32_t one[U] = {1u, 1u, 1u, 1u};
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const uint32_t i = i0 + k * STEP;
+            l[k] = i < n ? __ldcg(s + i) : 0u;
+            r[k] = i + 1u < n ? __ldcg(s + i + 1u) : WORD_START_BIT;
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            pair[k] = (l[k] & TOKEN_MASK) << 16 | (r[k] & TOKEN_MASK);
+            if (tail_counted(l[k], r[k])) wanted |= 1u << k;
+            if (copy && i0 + k * STEP < n) copy[i0 + k * STEP] = l[k];
+        }
+        wt_updates<U>(A, T, pair, one, wanted, rise ? 15u : 0u, tau);
+    }
+}
+// Phase 2 over [from, to): what is copied goes to dst[out...], and the source gets this merge's rewrite.
+__device__ __forceinline__ void tail_move(const TailView& v, uint32_t* src, uint32_t* __restrict__ dst, uint32_t from, uint32_t to, uint32_t out, uint32_t lane) {
+    for (uint32_t span = from; span < to; span += TAIL_SPAN) {
+        TailSpan t;
+        tail_span(v, span, lane, t);
+        if (span + TAIL_SPAN <= to && !__any_sync(0xFFFFFFFFu, t.match != 0u || t.left)) {
+            // nothing changes: whole 16-byte stores; element `shift` of every lane's four lies on a 16-byte boundary of the destination
+            const uint32_t shift = (0u - out) & 3u;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint4 a = t.q[u];
+                uint4 b;
+                b.x = __shfl_down_sync(0xFFFFFFFFu, a.x, 1); b.y = __shfl_down_sync(0xFFFFFFFFu, a.y, 1); b.z = __shfl_down_sync(0xFFFFFFFFu, a.z, 1);
+                const uint4 n0 = t.q[u < 3 ? u + 1 : u];
+                const uint32_t fx = __shfl_sync(0xFFFFFFFFu, n0.x, 0), fy = __shfl_sync(0xFFFFFFFFu, n0.y, 0), fz = __shfl_sync(0xFFFFFFFFu, n0.z, 0);
+                if (lane == 31) { b.x = fx; b.y = fy; b.z = fz; }
+                uint32_t* o = dst + out + u * 128u + lane * 4u;
+                if (u == 0 && lane == 0) { if (shift > 0u) o[0] = a.x; if (shift > 1u) o[1] = a.y; if (shift > 2u) o[2] = a.z; }
+                if (u == 3 && lane == 31 && shift) {      // what does not fill a store
+                    if (shift == 1u) o[1] = a.y;
+                    if (shift <= 2u) o[2] = a.z;
+                    o[3] = a.w;
+                } else {
+                    const uint4 w = shift == 0u ? a : shift == 1u ? make_uint4(a.y, a.z, a.w, b.x) : shift == 2u ? make_uint4(a.z, a.w, b.x, b.y)
+                                                                                                               : make_uint4(a.w, b.x, b.y, b.z);
+                    *reinterpret_cast<uint4*>(o + shift) = w;
+                }
+            }
+            out += TAIL_SPAN;
+            continue;
+        }
+        bool carry = t.left;          // the symbol before this lane's four is the first of a pair
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t i = span + u * 128u + lane * 4u, m = (t.match >> (4 * u)) & 15u;
+            uint32_t before = __shfl_up_sync(0xFFFFFFFFu, m >> 3, 1);
+            if (lane == 0) before = carry ? 1u : 0u;
+            carry = __shfl_sync(0xFFFFFFFFu, m >> 3, 31) != 0u;
+            const uint32_t sym[4] = {t.q[u].x, t.q[u].y, t.q[u].z, t.q[u].w};
+            const uint32_t keep = ~(m << 1 | before) & 15u;
+            const uint32_t there = i >= to ? 0u : to - i >= 4u ? 15u : (1u << (to - i)) - 1u;
+            const uint32_t below = (1u << lane) - 1u, copied = keep & there;
+            uint32_t at = out, row = 0u;
+#pragma unroll
+            for (int k = 0; k < 4; k++) { const uint32_t b = __ballot_sync(0xFFFFFFFFu, (copied >> k) & 1u); at += __popc(b & below); row += __popc(b); }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const bool mine = (m & there) >> k & 1u;
+                const uint32_t x = mine ? (sym[k] & WORD_START_BIT) | v.fresh : sym[k];
+                if (mine) src[i + k] = x;
+                if ((copied >> k) & 1u) dst[at++] = x;
+            }
+            out += row;
+        }
+    }
+}
+
+template <bool LITERAL>
 __global__ void __launch_bounds__(WM_THREADS, 1)
 k_word_merges(WordArgs A, uint32_t target) {
     extern __shared__ __align__(16) unsigned char wm_smem[];
@@ -349,11 +570,12 @@ k_word_merges(WordArgs A, uint32_t target) {
     __syncthreads();
     if (tid == 0) {
         s.queued = 0u; s.flags = 0u; s.inserted = 0u; s.ncand = s.init.tau == ~0ull ? 0u : nc;
-        s.c_entries = s.init.entries; s.c_inserted = 0u;
+        s.c_entries = s.init.entries; s.c_inserted = 0u; s.c_merged = 0u; s.tail_queued = 0u;
     }
     cluster_barrier();           // also: everybody has read the control block before anybody writes it
     uint32_t done = s.init.merges_done, next_id = s.init.next_id, symbols = s.init.symbols, scans = s.init.scans;
     uint32_t early = s.init.early_stop, status = s.init.status;
+    uint32_t front = s.init.front, front_before = s.init.front_before, turn = s.init.turn;
     unsigned long long tau = s.init.tau, best = s.init.best;
     bool valid = s.init.best_valid != 0u;
     uint32_t occ_most = s.init.occupied;     // upper bound of the occupied slots
@@ -381,12 +603,27 @@ k_word_merges(WordArgs A, uint32_t target) {
         const uint32_t len = end - beg;
         const uint32_t usual_a = a < 256u ? 1u : __ldcg(A.usual + a), usual_b = b < 256u ? 1u : __ldcg(A.usual + b);
         // a merge makes at most two new pairs per symbol in use, and per occurrence
-        const uint32_t grow = 2u * min(min(len, count), fresh + 1u);
+        // (the tail: at most two per copied occurrence, with the new symbol, and what the older symbols bring back)
+        const uint32_t grow = 2u * min(min(len, count), fresh + 1u) + (LITERAL ? 4u * min(count, fresh) + 4u : 0u);
         if (occ_most + grow > room) {
             occ_most = occ_start + T.lead->c_inserted;     // stable here: it changes between the two barriers of a merge
             if (occ_most + grow > room) { status = WS_GROW; break; }
         }
         occ_most += grow;
+        TailView tail{};
+        uint32_t* tail_src = nullptr;
+        uint32_t tail_from = 0u, tail_to = 0u;
+        if (LITERAL) {
+            tail_src = A.tail[turn % 3u];
+            const uint32_t n = symbols - front;
+            if (count >= n) { status = WS_TAIL; break; }
+            tail = TailView{tail_src, n, n - count, a, b, fresh};
+            // a warp's share of what is copied, in whole spans
+            const uint32_t share = (tail.limit + TAIL_SPAN * (STEP / 32u) - 1u) / (TAIL_SPAN * (STEP / 32u)) * TAIL_SPAN;
+            tail_from = min(tail.limit, (rank * (WM_THREADS / 32) + (tid >> 5)) * share);
+            tail_to = min(tail.limit, tail_from + share);
+        }
+        uint32_t merged = 0u;        // LITERAL: symbols of the text's front that this thread's occurrences drop
 
         // ── phase 1: occurrences, counts, the new symbol's list ──
         auto apply = [&](uint32_t qi) {
@@ -406,7 +643,9 @@ k_word_merges(WordArgs A, uint32_t target) {
             if (ok && !(rp & WP_START)) { l = p - wp_span(prev_end); rl = A.rec[l]; x = wp_sym(rl); }
             if (a == b && x == a) ok = false;         // inside a run of equal symbols: its first position merges the whole run
             uint32_t r = q + wp_span(rq), rr = !ok ? WP_START : r == r_usual ? rec_r : A.rec[r];
-            if (a == b) while (ok && !(rr & WP_START) && wp_sym(rr) == a) { r += wp_span(rr); rr = A.rec[r]; }
+            uint32_t drops = 1u;
+            if (a == b) while (ok && !(rr & WP_START) && wp_sym(rr) == a) { r += wp_span(rr); rr = A.rec[r]; drops++; }
+            if (LITERAL && ok) merged += drops * w;
             const uint32_t span = r - p;
             uint32_t y = (!ok || (rr & WP_START)) ? 0u : wp_sym(rr);
             uint32_t right_left = b;                   // symbol on the left of the right-hand neighbour before the merge
@@ -505,13 +744,57 @@ k_word_merges(WordArgs A, uint32_t target) {
         };
         static_assert(WM_THREADS * WM_UNROLL <= WM_QUEUE, "a round fits the queue");
         const bool spilled = walk(apply);
-        if (gtid == 0) {
+        if (LITERAL) {
+            merged = __reduce_add_sync(0xFFFFFFFFu, merged);
+            if (lane == 0 && merged) atomicAdd(&T.lead->c_merged, merged);
+            const uint32_t kept = tail_count(A, T, tail, tail_from, tail_to, tau);
+            tail_pairs(A, T, tail_src + (tail.limit - 1u), tail.n - (tail.limit - 1u), gtid, false, tau, nullptr);
+            if (lane == 0) s.wkept[tid >> 5] = kept;
+            __syncthreads();
+            for (uint32_t i = tid; i < min(s.tail_queued, TAIL_QUEUE); i += WM_THREADS) tail_match_changes(A, T, tail, s.tail_queue[i], tau);
+            if (tid < 32) {
+                const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, tid < WM_THREADS / 32 ? s.wkept[tid] : 0u);
+                if (tid < WM_CLUSTER) cluster.map_shared_rank(&s, tid)->xkept[rank] = all;
+            }
+        } else if (gtid == 0) {
             // every occurrence of the pair itself goes
             wt_update(A, T, pair, count, false, tau);
         }
         __syncwarp();
         cluster_barrier();
 
+        uint32_t dropped = 0u, kept_all = 0u, stale = 0u;      // LITERAL: see below
+        if (LITERAL) {
+            dropped = T.lead->c_merged;                        // by the front; the rest of `count` by the tail
+            uint32_t kept = lane < WM_CLUSTER ? s.xkept[lane] : 0u, out = lane < rank ? kept : 0u;
+            kept_all = __reduce_add_sync(0xFFFFFFFFu, kept);
+            out = __reduce_add_sync(0xFFFFFFFFu, out + (lane < (tid >> 5) ? s.wkept[lane] : 0u));
+            const uint32_t n1 = tail.n - (count - dropped);    // tail symbols after this merge, kept_all of them copied
+            stale = n1 - kept_all;
+            const uint32_t from = front - dropped + kept_all;  // position of the first that keeps its older contents
+            if (stale && from < front_before) { status = WS_TAIL; break; }
+            uint32_t* dst = A.tail[(turn + 1u) % 3u];
+            const uint32_t* older = A.tail[(turn + 2u) % 3u] + (from - front_before);
+            tail_move(tail, tail_src, dst, tail_from, tail_to, out, lane);
+            for (uint32_t i = tail.limit + gtid; i < tail.n; i += STEP) {       // the rewrite where nothing is copied
+                const uint32_t l = tail_at(tail, i);
+                if (tail_match(tail, l, tail_at(tail, i + 1u))) tail_src[i] = (l & WORD_START_BIT) | fresh;
+            }
+            tail_pairs(A, T, older, stale, gtid, true, tau, dst + kept_all);
+            if (gtid == 0) {
+                if (stale) {      // the last copied symbol and the first older one
+                    uint32_t i = tail.limit - 1u, l = tail_at(tail, i);
+                    while (i > 0u && tail_match(tail, tail_at(tail, i - 1u), l)) l = tail_at(tail, --i);
+                    if (tail_match(tail, l, tail_at(tail, i + 1u))) l = fresh;
+                    const uint32_t r = __ldcg(older);
+                    if (tail_counted(l, r)) tail_pair(A, T, l, r, true, tau);
+                }
+                if (dropped) {    // the front's occurrences of the pair itself go (the tail's went one by one)
+                    wt_update(A, T, pair, dropped, false, tau);
+                }
+            }
+            __syncwarp();
+        }
         // ── phase 2: the records; the next merge's pair ──
         if (!spilled) {
             const uint32_t n = s.queued;
@@ -546,6 +829,7 @@ k_word_merges(WordArgs A, uint32_t target) {
             s.init.entries = e1;
             A.log[done] = make_uint4(a, b, fresh, count);
         }
+        if (LITERAL) cluster_barrier();      // counts change in phase 2 too: all of them before the arg-max looks
         if (tid == 0 && s.inserted) {
             atomicAdd(&T.lead->c_inserted, s.inserted);
             s.inserted = 0u;
@@ -553,6 +837,13 @@ k_word_merges(WordArgs A, uint32_t target) {
         done++;
         next_id++;
         symbols -= count;
+        if (LITERAL) {
+            front_before = front;
+            front -= dropped;
+            turn++;
+            if (gtid == 0) s.c_merged = 0u;
+            if (tid == 0) s.tail_queued = 0u;
+        }
         word_argmax(A, T, best, flags);
         if (flags & WS_FULL) { status = WS_FULL; break; }
     }
@@ -573,6 +864,9 @@ k_word_merges(WordArgs A, uint32_t target) {
         o.occupied = occ_start + s.c_inserted;
         o.symbols = symbols;
         o.scans = scans;
+        o.front = front;
+        o.front_before = front_before;
+        o.turn = turn;
         *A.st = o;
     }
     cluster_barrier();           // no CTA ends while its shared memory may still be read

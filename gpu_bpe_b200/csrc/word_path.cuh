@@ -30,6 +30,12 @@ struct WordPath {
     uint4* h_log = nullptr;              // pinned
     uint32_t goal = 0;                   // merges the log has room for
     bool given_log2 = false;             // the caller chose the pair table's size
+    bool literal = false;
+    uint64_t n_front = 0;                // bytes that the dictionary takes: all, or what is before the tail of a "literal" run
+    uint64_t cap_tail = 0;
+    static constexpr uint32_t TAIL_SHORT = 3, TAIL_LONG = 8;
+    uint32_t tail_share = TAIL_SHORT;    // 32nds of the text
+    WordState seen{};                    // control block after the last batch
     uint64_t launches = 0;
     std::vector<cudaEvent_t> ev;
 
@@ -41,7 +47,7 @@ struct WordPath {
         for (void* p : {(void*)dict.short_key, (void*)dict.short_cnt, (void*)dict.short_base, (void*)dict.long_key, (void*)dict.long_cnt,
                         (void*)dict.long_base, (void*)dict.st, (void*)args.rec, (void*)args.weight, (void*)args.byte_list, (void*)args.byte_off,
                         (void*)args.entries, (void*)args.segment, (void*)args.usual, (void*)args.table, (void*)args.cand, (void*)args.st, (void*)args.log,
-                        (void*)cursor, (void*)bins, (void*)own_mask, (void*)own_bytes})
+                        (void*)cursor, (void*)bins, (void*)own_mask, (void*)own_bytes, (void*)args.tail[0], (void*)args.tail[1], (void*)args.tail[2]})
             ctx->free(p);
         if (h_state) cudaFreeHost(h_state);
         for (auto e : ev) cudaEventDestroy(e);
@@ -49,9 +55,10 @@ struct WordPath {
     }
 
     // Buffers whose size does not depend on the text.
-    b200bpe_status create(Ctx* c, uint64_t n_bytes, uint32_t merges_goal, uint32_t table_log2) {
+    b200bpe_status create(Ctx* c, uint64_t n_bytes, uint32_t merges_goal, uint32_t table_log2, bool literal_mode) {
         ctx = c;
         n = n_bytes;
+        literal = literal_mode;
         goal = std::max<uint32_t>(1, merges_goal);
         auto log2_of = [](uint64_t x) { uint32_t l = 0; while ((1ull << l) < x) l++; return l; };
         // slots for one distinct short word per 8 bytes and one distinct long word per 32
@@ -84,14 +91,18 @@ struct WordPath {
             ev.push_back(e);
         }
         B2_CUDA(cudaFuncSetAttribute(k_dict_words, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WD_SMEM_BYTES));
-        B2_CUDA(cudaFuncSetAttribute(k_word_merges, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WordShared)));
-        B2_CUDA(cudaFuncSetAttribute(k_word_merges, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        B2_CUDA(cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WordShared)));
+        B2_CUDA(cudaFuncSetAttribute(kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         return B200BPE_OK;
     }
 
     int blocks(uint64_t items, int per_block, int per_sm) const {
         return (int)std::max<uint64_t>(1, std::min<uint64_t>((items + per_block - 1) / per_block, (uint64_t)ctx->sm_count * per_sm));
     }
+    void (*kernel() const)(WordArgs, uint32_t) { return literal ? k_word_merges<true> : k_word_merges<false>; }
+    // The tail has to hold about three times a merge's count: what is dropped, and what came in its place two merges ago.  The first
+    // merges count most, some 2.5 % of a text each; a run that they end starts again with a longer tail.
+    uint64_t tail_goal() const { return n / 32 * tail_share; }
     int aligned() const { return (((uintptr_t)bytes | (uintptr_t)mask) & 15u) == 0 ? 1 : 0; }
 
     // Builds the dictionary of the text and the state of a fresh run.  *fits is false (and nothing else is set up) when the text is
@@ -119,9 +130,18 @@ struct WordPath {
         B2_CUDA(cudaMemsetAsync(dict.short_cnt, 0, sizeof(uint32_t) << dict.short_log2, s));
         B2_CUDA(cudaMemsetAsync(dict.long_key, 0, sizeof(unsigned long long) << dict.long_log2, s));
         B2_CUDA(cudaMemsetAsync(dict.long_cnt, 0, sizeof(uint32_t) << dict.long_log2, s));
-        k_dict_words<<<blocks(n, WD_TILE, 3), WD_THREADS, WD_SMEM_BYTES, s>>>(bytes, mask, n, dict, aligned());
+        n_front = n;
+        if (literal) {
+            k_dict_split_at<<<1, 256, 0, s>>>(mask, n, n - tail_goal(), dict.st);
+            launches++;
+            B2_CUDA(cudaMemcpyAsync(h_dict, dict.st, sizeof(DictState), cudaMemcpyDeviceToHost, s));
+            B2_CUDA(cudaStreamSynchronize(s));
+            n_front = h_dict->split;
+            if (n_front == 0 || n_front >= n) return B200BPE_OK;
+        }
+        k_dict_words<<<blocks(n_front, WD_TILE, 3), WD_THREADS, WD_SMEM_BYTES, s>>>(bytes, mask, n_front, dict, aligned());
         const uint64_t slots = (1ull << dict.short_log2) + (1ull << dict.long_log2);
-        k_dict_places<<<blocks(slots, 1024, 8), 256, 0, s>>>(mask, n, dict);
+        k_dict_places<<<blocks(slots, 1024, 8), 256, 0, s>>>(mask, n_front, dict);
         launches += 2;
         B2_CUDA(cudaMemcpyAsync(h_dict, dict.st, sizeof(DictState), cudaMemcpyDeviceToHost, s));
         B2_CUDA(cudaStreamSynchronize(s));
@@ -143,8 +163,20 @@ struct WordPath {
         uint32_t* off = const_cast<uint32_t*>(args.byte_off);
         B2_CUDA(cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 65536, s));
         B2_CUDA(cudaMemsetAsync(args.st, 0, sizeof(WordState), s));
-        k_dict_fill<<<blocks(slots, 256, 16), 256, 0, s>>>(bytes, mask, n, dict, args.rec, weight);
+        k_dict_fill<<<blocks(slots, 256, 16), 256, 0, s>>>(bytes, mask, n_front, dict, args.rec, weight);
         k_dict_count<<<blocks(positions, 256, 8), 256, 0, s>>>(args.rec, weight, positions, bins);
+        if (literal) {
+            const uint64_t tail = n - n_front;
+            if (tail > cap_tail) {
+                for (auto& t : args.tail) { ctx->free(t); t = nullptr; }
+                for (auto& t : args.tail) B2_CUDA(ctx->alloc(&t, sizeof(uint32_t) * (tail + 4)));
+                cap_tail = tail;
+            }
+            // (the destination of the first merge starts zeroed, as a fresh WebGPU buffer does: it is what the older symbols come from)
+            B2_CUDA(cudaMemsetAsync(args.tail[2], 0, sizeof(uint32_t) * tail, s));
+            k_dict_tail<<<blocks(tail, 256, 16), 256, 0, s>>>(bytes, mask, n_front, n, args.tail[0], bins);
+            launches++;
+        }
         k_dict_offsets<<<1, 1024, 0, s>>>(bins, off, cursor, dict.st);
         k_dict_lists<<<blocks(positions, 256, 8), 256, 0, s>>>(args.rec, positions, cursor, list);
         launches += 4;
@@ -152,10 +184,10 @@ struct WordPath {
         // at most): a probe that collides is another round trip, and the scans that pay for its size are a few in a run.
         if (args.table_log2 == 0) {
             uint32_t l = 13;
-            while (l < 23 && (2ull << l) < positions) l++;
+            while (l < 23 && (2ull << l) < positions + (n - n_front)) l++;
             args.table_log2 = l;
         }
-        uint64_t most = std::min<uint64_t>(positions, 65536);
+        uint64_t most = std::min<uint64_t>((uint64_t)positions + (n - n_front), 65536);
         if (given_log2) {   // a size from the caller holds what there is, and no more
             B2_CUDA(cudaMemcpyAsync(h_dict, dict.st, sizeof(DictState), cudaMemcpyDeviceToHost, s));
             B2_CUDA(cudaStreamSynchronize(s));
@@ -167,7 +199,10 @@ struct WordPath {
         }
         if (!args.table) B2_CUDA(ctx->alloc(&args.table, sizeof(unsigned long long) << args.table_log2));
         B2_CUDA(cudaMemsetAsync(args.table, 0, sizeof(unsigned long long) << args.table_log2, s));
-        k_word_init<<<256, 256, 0, s>>>(bins, dict.st, args.table, args.table_log2, args.st, first_id, (uint32_t)n);
+        k_word_init<<<256, 256, 0, s>>>(bins, dict.st, args.table, args.table_log2, args.st, first_id, (uint32_t)n, (uint32_t)n_front);
+        seen = WordState{};
+        seen.symbols = (uint32_t)n;
+        seen.front = (uint32_t)n_front;
         launches++;
         B2_CUDA(cudaGetLastError());
         *fits = true;
@@ -186,7 +221,7 @@ struct WordPath {
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        B2_CUDA(cudaLaunchKernelEx(&cfg, k_word_merges, args, target));
+        B2_CUDA(cudaLaunchKernelEx(&cfg, kernel(), args, target));
         launches++;
         return B200BPE_OK;
     }
@@ -210,13 +245,15 @@ struct WordPath {
     // The live symbols into d_out (device, room for the count in `symbols`).
     b200bpe_status expand(uint32_t* d_out) {
         cudaStream_t s = ctx->stream;
-        const uint64_t tiles = (n + WD_TILE - 1) / WD_TILE;
+        const uint64_t tiles = (n_front + WD_TILE - 1) / WD_TILE;
         uint32_t* counts = nullptr;
         B2_CUDA(ctx->alloc(&counts, sizeof(uint32_t) * (tiles + 1)));
-        k_dict_expand<false><<<blocks(tiles, 1, 4), WD_THREADS, 0, s>>>(bytes, mask, n, dict, args.rec, counts, nullptr, aligned());
+        k_dict_expand<false><<<blocks(tiles, 1, 4), WD_THREADS, 0, s>>>(bytes, mask, n_front, dict, args.rec, counts, nullptr, aligned());
         k_dict_scan<<<1, 1024, 0, s>>>(counts, tiles);
-        k_dict_expand<true><<<blocks(tiles, 1, 4), WD_THREADS, 0, s>>>(bytes, mask, n, dict, args.rec, counts, d_out, aligned());
+        k_dict_expand<true><<<blocks(tiles, 1, 4), WD_THREADS, 0, s>>>(bytes, mask, n_front, dict, args.rec, counts, d_out, aligned());
         launches += 3;
+        if (n_front < n)
+            B2_CUDA(cudaMemcpyAsync(d_out + seen.front, args.tail[seen.turn % 3], sizeof(uint32_t) * (size_t)(seen.symbols - seen.front), cudaMemcpyDeviceToDevice, s));
         cudaError_t e = cudaGetLastError();
         ctx->free(counts);
         B2_CUDA(e);
