@@ -22,6 +22,7 @@ class TrieTokenizer:
         options = options or {}
         self._engine = engine
         self._vocab = vocab if vocab is not None else [[i] for i in range(256)]
+        self._dh = self._decode_entries = None
         header = parseHeader(trieData)   # raises the reference's errors for bad magic / version / length
         buf = np.frombuffer(trieData, np.uint8)
         h = C.c_void_p()
@@ -101,7 +102,40 @@ class TrieTokenizer:
         _lib.lib().b200bpe_tokenizer_last_ms(self._h, C.byref(a), C.byref(b))
         return a.value, b.value
 
+    def _decoder(self):
+        """Handle that decodes the vocabulary as it is now, or None where the general way has to do it: entries other than bytes
+        objects (they could change under the handle), a destroyed tokenizer or engine."""
+        if self._h is None or self._engine._ctx is None or not isinstance(self._vocab, list):
+            return None
+        try:
+            same = self._decode_entries is not None and self._decode_entries == self._vocab
+        except ValueError:            # (entries that compare element by element)
+            same = False
+        if not same:
+            self._drop_decoder()
+            if set(map(type, self._vocab)) == {bytes}:
+                self._decode_entries = list(self._vocab)
+                blob = np.frombuffer(b"".join(self._decode_entries) or b"\0", np.uint8)
+                off = np.zeros(len(self._decode_entries) + 1, np.uint64)
+                np.cumsum(np.fromiter(map(len, self._decode_entries), np.uint64, len(self._decode_entries)), out=off[1:])
+                h = C.c_void_p()
+                if _lib.lib().b200bpe_decoder_create(self._engine.ctx, blob.ctypes.data, off.ctypes.data, off.size - 1, C.byref(h)) == 0:
+                    self._dh = h
+        return self._dh
+
+    def _drop_decoder(self):
+        if self._dh is not None:
+            _lib.lib().b200bpe_decoder_destroy(self._dh)
+        self._dh = self._decode_entries = None
+
     def decode(self, tokens) -> bytes:
+        if isinstance(tokens, np.ndarray) and tokens.dtype == np.uint32 and tokens.ndim == 1 and tokens.size and self._decoder() is not None:
+            t = np.ascontiguousarray(tokens)
+            n = C.c_uint64()
+            if _lib.lib().b200bpe_decoder_run(self._dh, t.ctypes.data, t.size, C.byref(n)) == 0:
+                text = np.empty(n.value, np.uint8)
+                _lib.check(_lib.lib().b200bpe_decoder_read(self._dh, text.ctypes.data, text.size), "b200bpe_decoder_read")
+                return text.tobytes()
         out = bytearray()
         for t in tokens:
             t = int(t)
@@ -109,6 +143,8 @@ class TrieTokenizer:
         return bytes(out)
 
     def destroy(self):
+        if self._engine._ctx is not None:
+            self._drop_decoder()
         if self._h is not None:
             _lib.lib().b200bpe_tokenizer_destroy(self._h)
             self._h = None

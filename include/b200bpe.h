@@ -242,6 +242,15 @@ b200bpe_status b200bpe_encode_device_noalloc(b200bpe_tok*, const uint8_t* d_byte
 b200bpe_status b200bpe_tokenizer_last_ms(b200bpe_tok*, double* walk_ms, double* compact_ms);
 void b200bpe_tokenizer_destroy(b200bpe_tok*);
 
+/* Token ids back to bytes (TrieTokenizer.decode, src/bpe/tokenizer/tokenizer.js): entry t of the vocabulary is bytes[offsets[t]] up to
+ * bytes[offsets[t + 1]]; an id of n_entries or more gives U+FFFD.  _run decodes host tokens into a device buffer of the handle and says how
+ * many bytes that made, _read copies them to the host.  One call at a time per handle. */
+typedef struct b200bpe_decoder b200bpe_decoder;
+b200bpe_status b200bpe_decoder_create(b200bpe_ctx*, const uint8_t* bytes, const uint64_t* offsets, uint32_t n_entries, b200bpe_decoder** out);
+b200bpe_status b200bpe_decoder_run(b200bpe_decoder*, const uint32_t* tokens, uint64_t n, uint64_t* n_bytes_out);
+b200bpe_status b200bpe_decoder_read(b200bpe_decoder*, uint8_t* out, uint64_t cap);
+void b200bpe_decoder_destroy(b200bpe_decoder*);
+
 /* ── merge-replay encoding: replaces TokenizerManager.encode (src/ui/tokenizer-manager.js:13-61) ──
  * The reference's other encoder: one token per byte, then every merge rule {a, b, new_id} applied in the order
  * it was learned, each as one left-to-right pass over the whole token list (no word boundaries, no chunks; with
