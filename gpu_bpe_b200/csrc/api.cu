@@ -146,6 +146,7 @@ void b200bpe_ctx_destroy(b200bpe_ctx* c) {
     if (c->c.comm && c->c.nccl.CommDestroy) c->c.nccl.CommDestroy(c->c.comm);
     if (c->c.stream) cudaStreamDestroy(c->c.stream);
     if (c->c.pool) cudaMemPoolDestroy(c->c.pool);
+    for (const auto& b : c->c.pinned) cudaFreeHost(b.p);
     delete c;
 }
 

@@ -1,7 +1,9 @@
 // Context object: one GPU, one stream, optional NCCL communicator for sharded jobs.
 #pragma once
 
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "common.cuh"
 
@@ -45,6 +47,37 @@ struct Ctx {
         return e;
     }
     void free(void* p) { if (p) cudaFreeAsync(p, stream); }
+    // Pinned host memory of this context's short-lived objects: cudaMallocHost takes 3 to 5 ms, half of a training call on a page of
+    // text.  A few blocks are kept between objects, PINNED_KEEP bytes at most, and go with the context.  A block is only given back when no
+    // copy to or from it is on its way.
+    struct Pinned { void* p; size_t bytes; };
+    std::vector<Pinned> pinned;
+    std::mutex pinned_mutex;
+    static constexpr size_t PINNED_KEEP = 4u << 20, PINNED_BLOCKS = 8;
+    cudaError_t alloc_pinned(void** p, size_t* bytes) {     // *bytes: wanted, then what the block has
+        {
+            std::lock_guard<std::mutex> lock(pinned_mutex);
+            for (size_t i = 0; i < pinned.size(); i++)
+                if (pinned[i].bytes >= *bytes) {
+                    *p = pinned[i].p;
+                    *bytes = pinned[i].bytes;
+                    pinned.erase(pinned.begin() + (ptrdiff_t)i);
+                    return cudaSuccess;
+                }
+        }
+        *bytes = (*bytes + 0xFFFFu) & ~(size_t)0xFFFFu;
+        return cudaMallocHost(p, *bytes);
+    }
+    void free_pinned(void* p, size_t bytes) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lock(pinned_mutex);
+            size_t kept = bytes;
+            for (const Pinned& b : pinned) kept += b.bytes;
+            if (pinned.size() < PINNED_BLOCKS && kept <= PINNED_KEEP) { pinned.push_back({p, bytes}); return; }
+        }
+        cudaFreeHost(p);
+    }
 };
 
 b200bpe_status load_nccl(const char* path, NcclApi* api);

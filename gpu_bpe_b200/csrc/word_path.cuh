@@ -25,6 +25,7 @@ struct WordPath {
     uint32_t positions = 0;
     WordState* h_state = nullptr;        // pinned: one per batch in flight
     DictState* h_dict = nullptr;         // pinned
+    size_t pinned = 0;                   // bytes of the pinned block
     uint8_t* own_mask = nullptr;         // heuristic word starts, or those of tagged symbols
     uint8_t* own_bytes = nullptr;
     uint4* h_log = nullptr;              // pinned
@@ -49,7 +50,7 @@ struct WordPath {
                         (void*)args.entries, (void*)args.segment, (void*)args.usual, (void*)args.table, (void*)args.cand, (void*)args.st, (void*)args.log,
                         (void*)cursor, (void*)bins, (void*)own_mask, (void*)own_bytes, (void*)args.tail[0], (void*)args.tail[1], (void*)args.tail[2]})
             ctx->free(p);
-        if (h_state) cudaFreeHost(h_state);
+        ctx->free_pinned(h_state, pinned);
         for (auto e : ev) cudaEventDestroy(e);
         ctx = nullptr;
     }
@@ -81,8 +82,8 @@ struct WordPath {
         B2_CUDA(ctx->alloc(&args.cand, sizeof(uint32_t) * WM_CLUSTER * (WM_CAND + 1)));
         B2_CUDA(ctx->alloc(&args.st, sizeof(WordState)));
         B2_CUDA(ctx->alloc(&args.log, sizeof(uint4) * (size_t)goal));
-        const size_t pinned = sizeof(WordState) * IN_FLIGHT + sizeof(DictState) + sizeof(uint4) * (size_t)goal;
-        B2_CUDA(cudaMallocHost(&h_state, pinned));
+        pinned = sizeof(WordState) * IN_FLIGHT + sizeof(DictState) + sizeof(uint4) * (size_t)goal;
+        B2_CUDA(ctx->alloc_pinned(reinterpret_cast<void**>(&h_state), &pinned));
         h_log = reinterpret_cast<uint4*>(h_state + IN_FLIGHT);
         h_dict = reinterpret_cast<DictState*>(h_log + goal);
         for (int i = 0; i < IN_FLIGHT; i++) {
