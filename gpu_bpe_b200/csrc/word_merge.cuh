@@ -77,7 +77,7 @@ struct WordShared {
     unsigned long long wbest[WM_THREADS / 32];
     uint32_t queued, ncand, flags, inserted;
     uint32_t c_entries, c_inserted, c_merged;   // the cluster's counters: those of CTA 0 are the ones in use
-    uint32_t xkept[WM_CLUSTER], wkept[WM_THREADS / 32];   // tail symbols that a CTA, a warp copies
+    uint32_t kept[WM_CLUSTER * WM_THREADS / 32];          // tail symbols that every warp of the cluster copies
     uint32_t tail_queue[4096], tail_queued;               // matches in this CTA's part of the tail
     WordState init;
 };
@@ -347,6 +347,9 @@ __device__ __noinline__ void word_scan(const WordArgs& A, WordTeam& T, unsigned 
 // A merge reads the tail twice: phase 1 counts what every warp's share keeps and updates the pairs that change; phase 2, with every
 // offset known, writes the destination, rewrites the source in place as the reference does (train.wgsl:486-487: the next merge but one may see it),
 // and copies the older symbols in.  The pairs' counts can rise here at any time, unlike the dictionary's.
+// What bounds it: the round trip of a span's loads (the next span's are on their way meanwhile) and, where matches are many, the updates of
+// the pairs around them.  Whole runs, us a merge: 64 KiB 15.5 -> 14.3, 1 MiB 17.3 -> 15.3 with the next span fetched ahead, shares dealt
+// round the CTAs and the tail's matches worked on beside the dictionary's; on the symbol buffers 36 and 31.
 struct TailView {
     const uint32_t* cur;
     uint32_t n, limit;           // its symbols; the first `limit` are copied
@@ -412,8 +415,8 @@ __device__ __forceinline__ void tail_match_changes(const WordArgs& A, WordTeam& 
 // u-th four; left: one begins right before the span.
 constexpr uint32_t TAIL_SPAN = 512;
 constexpr uint32_t TAIL_QUEUE = 4096;
-struct TailSpan { uint4 q[4]; uint32_t match; bool left; };
-__device__ __forceinline__ void tail_span(const TailView& v, uint32_t base, uint32_t lane, TailSpan& t) {
+struct TailSpan { uint4 q[4]; uint32_t edge, match; bool left; };
+__device__ __forceinline__ void tail_fetch(const TailView& v, uint32_t base, uint32_t lane, TailSpan& t) {
     if (base + TAIL_SPAN <= v.limit) {          // (behind the limit the rewrite is under way in phase 2)
         const uint4* __restrict__ p = reinterpret_cast<const uint4*>(v.cur + base) + lane;
 #pragma unroll
@@ -425,9 +428,11 @@ __device__ __forceinline__ void tail_span(const TailView& v, uint32_t base, uint
             t.q[u] = make_uint4(tail_at(v, i), tail_at(v, i + 1u), tail_at(v, i + 2u), tail_at(v, i + 3u));
         }
     }
-    uint32_t edge = 0u;
-    if (lane < 2u) edge = lane == 0u ? (base > 0u ? tail_at(v, base - 1u) : WORD_START_BIT) : tail_at(v, base + TAIL_SPAN);
-    const uint32_t before = __shfl_sync(0xFFFFFFFFu, edge, 0), behind = __shfl_sync(0xFFFFFFFFu, edge, 1);
+    t.edge = 0u;
+    if (lane < 2u) t.edge = lane == 0u ? (base > 0u ? tail_at(v, base - 1u) : WORD_START_BIT) : tail_at(v, base + TAIL_SPAN);
+}
+__device__ __forceinline__ void tail_decide(const TailView& v, uint32_t lane, TailSpan& t) {
+    const uint32_t before = __shfl_sync(0xFFFFFFFFu, t.edge, 0), behind = __shfl_sync(0xFFFFFFFFu, t.edge, 1);
     t.match = 0u;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
@@ -443,9 +448,12 @@ __device__ __forceinline__ void tail_span(const TailView& v, uint32_t base, uint
 __device__ __forceinline__ uint32_t tail_count(const WordArgs& A, WordTeam& T, const TailView& v, uint32_t from, uint32_t to, unsigned long long tau) {
     const uint32_t lane = T.tid & 31;
     uint32_t kept = to - from;
+    TailSpan t, ahead;               // the next span is on its way while this one is worked on
+    if (from < to) tail_fetch(v, from, lane, ahead);
     for (uint32_t span = from; span < to; span += TAIL_SPAN) {
-        TailSpan t;
-        tail_span(v, span, lane, t);
+        t = ahead;
+        if (span + TAIL_SPAN < to) tail_fetch(v, span + TAIL_SPAN, lane, ahead);
+        tail_decide(v, lane, t);
         const uint32_t end = to - span;           // symbols of the span that are in question
         uint32_t match = t.match, drops = 0u;
         if (end < TAIL_SPAN) {
@@ -496,9 +504,12 @@ __device__ __forceinline__ void tail_pairs(const WordArgs& A, WordTeam& T, const
 }
 // Phase 2 over [from, to): what is copied goes to dst[out...], and the source gets this merge's rewrite.
 __device__ __forceinline__ void tail_move(const TailView& v, uint32_t* src, uint32_t* __restrict__ dst, uint32_t from, uint32_t to, uint32_t out, uint32_t lane) {
+    TailSpan t, ahead;
+    if (from < to) tail_fetch(v, from, lane, ahead);
     for (uint32_t span = from; span < to; span += TAIL_SPAN) {
-        TailSpan t;
-        tail_span(v, span, lane, t);
+        t = ahead;
+        if (span + TAIL_SPAN < to) tail_fetch(v, span + TAIL_SPAN, lane, ahead);
+        tail_decide(v, lane, t);
         if (span + TAIL_SPAN <= to && !__any_sync(0xFFFFFFFFu, t.match != 0u || t.left)) {
             // nothing changes: whole 16-byte stores; element `shift` of every lane's four lies on a 16-byte boundary of the destination
             const uint32_t shift = (0u - out) & 3u;
@@ -620,7 +631,7 @@ k_word_merges(WordArgs A, uint32_t target) {
             tail = TailView{tail_src, n, n - count, a, b, fresh};
             // a warp's share of what is copied, in whole spans
             const uint32_t share = (tail.limit + TAIL_SPAN * (STEP / 32u) - 1u) / (TAIL_SPAN * (STEP / 32u)) * TAIL_SPAN;
-            tail_from = min(tail.limit, (rank * (WM_THREADS / 32) + (tid >> 5)) * share);
+            tail_from = min(tail.limit, ((tid >> 5) * WM_CLUSTER + rank) * share);      // (neighbouring shares in different SMs)
             tail_to = min(tail.limit, tail_from + share);
         }
         uint32_t merged = 0u;        // LITERAL: symbols of the text's front that this thread's occurrences drop
@@ -743,19 +754,19 @@ k_word_merges(WordArgs A, uint32_t target) {
             return spilled;
         };
         static_assert(WM_THREADS * WM_UNROLL <= WM_QUEUE, "a round fits the queue");
+        if (LITERAL) {
+            const uint32_t kept = tail_count(A, T, tail, tail_from, tail_to, tau);
+            if (lane < WM_CLUSTER) cluster.map_shared_rank(&s, lane)->kept[(tid >> 5) * WM_CLUSTER + rank] = kept;
+            __syncthreads();
+        }
         const bool spilled = walk(apply);
         if (LITERAL) {
+            // the tail's matches from the last thread down: where both are few, other warps than those with the dictionary's occurrences
+            for (uint32_t i = WM_THREADS - 1u - tid; i < min(s.tail_queued, TAIL_QUEUE); i += WM_THREADS) tail_match_changes(A, T, tail, s.tail_queue[i], tau);
+            tail_pairs(A, T, tail_src + (tail.limit - 1u), tail.n - (tail.limit - 1u), gtid, false, tau, nullptr);
+            __syncwarp();
             merged = __reduce_add_sync(0xFFFFFFFFu, merged);
             if (lane == 0 && merged) atomicAdd(&T.lead->c_merged, merged);
-            const uint32_t kept = tail_count(A, T, tail, tail_from, tail_to, tau);
-            tail_pairs(A, T, tail_src + (tail.limit - 1u), tail.n - (tail.limit - 1u), gtid, false, tau, nullptr);
-            if (lane == 0) s.wkept[tid >> 5] = kept;
-            __syncthreads();
-            for (uint32_t i = tid; i < min(s.tail_queued, TAIL_QUEUE); i += WM_THREADS) tail_match_changes(A, T, tail, s.tail_queue[i], tau);
-            if (tid < 32) {
-                const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, tid < WM_THREADS / 32 ? s.wkept[tid] : 0u);
-                if (tid < WM_CLUSTER) cluster.map_shared_rank(&s, tid)->xkept[rank] = all;
-            }
         } else if (gtid == 0) {
             // every occurrence of the pair itself goes
             wt_update(A, T, pair, count, false, tau);
@@ -766,9 +777,15 @@ k_word_merges(WordArgs A, uint32_t target) {
         uint32_t dropped = 0u, kept_all = 0u, stale = 0u;      // LITERAL: see below
         if (LITERAL) {
             dropped = T.lead->c_merged;                        // by the front; the rest of `count` by the tail
-            uint32_t kept = lane < WM_CLUSTER ? s.xkept[lane] : 0u, out = lane < rank ? kept : 0u;
-            kept_all = __reduce_add_sync(0xFFFFFFFFu, kept);
-            out = __reduce_add_sync(0xFFFFFFFFu, out + (lane < (tid >> 5) ? s.wkept[lane] : 0u));
+            uint32_t out = 0u;                                 // what the warps with earlier shares copy
+#pragma unroll
+            for (uint32_t k = 0; k < WM_CLUSTER * WM_THREADS / 32; k += 32) {
+                const uint32_t kept = s.kept[k + lane];
+                kept_all += kept;
+                if (k + lane < (tid >> 5) * WM_CLUSTER + rank) out += kept;
+            }
+            kept_all = __reduce_add_sync(0xFFFFFFFFu, kept_all);
+            out = __reduce_add_sync(0xFFFFFFFFu, out);
             const uint32_t n1 = tail.n - (count - dropped);    // tail symbols after this merge, kept_all of them copied
             stale = n1 - kept_all;
             const uint32_t from = front - dropped + kept_all;  // position of the first that keeps its older contents
