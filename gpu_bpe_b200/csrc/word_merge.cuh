@@ -348,8 +348,8 @@ __device__ __noinline__ void word_scan(const WordArgs& A, WordTeam& T, unsigned 
 // offset known, writes the destination, rewrites the source in place as the reference does (train.wgsl:486-487: the next merge but one may see it),
 // and copies the older symbols in.  The pairs' counts can rise here at any time, unlike the dictionary's.
 // What bounds it: the round trip of a span's loads (the next span's are on their way meanwhile) and, where matches are many, the updates of
-// the pairs around them.  Whole runs, us a merge: 64 KiB 15.5 -> 14.3, 1 MiB 17.3 -> 15.3 with the next span fetched ahead, shares dealt
-// round the CTAs and the tail's matches worked on beside the dictionary's; on the symbol buffers 36 and 31.
+// the pairs around them.  Whole runs, us a merge: 64 KiB 15.5 -> 11.0, 1 MiB 17.3 -> 12.1 with the next span fetched ahead, shares dealt
+// round the CTAs, and matches and single updates worked on beside the dictionary's occurrences; on the symbol buffers 36 and 31.
 struct TailView {
     const uint32_t* cur;
     uint32_t n, limit;           // its symbols; the first `limit` are copied
@@ -573,6 +573,7 @@ k_word_merges(WordArgs A, uint32_t target) {
     WordTeam T{s, cluster.map_shared_rank(&s, 0), rank, tid, cluster};
     constexpr uint32_t STEP = WM_THREADS * WM_CLUSTER;
     const uint32_t gtid = tid * WM_CLUSTER + rank;        // neighbours in a list go to different SMs
+    const uint32_t gtid_mid = (tid ^ (WM_THREADS / 2)) * WM_CLUSTER + rank;   // the same from the middle: short lists side by side
 
     if (tid < sizeof(WordState) / 4) reinterpret_cast<uint32_t*>(&s.init)[tid] = __ldcg(reinterpret_cast<const uint32_t*>(A.st) + tid);
     uint32_t* my_cand = A.cand + (size_t)rank * (WM_CAND + 1);
@@ -763,12 +764,12 @@ k_word_merges(WordArgs A, uint32_t target) {
         if (LITERAL) {
             // the tail's matches from the last thread down: where both are few, other warps than those with the dictionary's occurrences
             for (uint32_t i = WM_THREADS - 1u - tid; i < min(s.tail_queued, TAIL_QUEUE); i += WM_THREADS) tail_match_changes(A, T, tail, s.tail_queue[i], tau);
-            tail_pairs(A, T, tail_src + (tail.limit - 1u), tail.n - (tail.limit - 1u), gtid, false, tau, nullptr);
+            tail_pairs(A, T, tail_src + (tail.limit - 1u), tail.n - (tail.limit - 1u), gtid_mid, false, tau, nullptr);
             __syncwarp();
             merged = __reduce_add_sync(0xFFFFFFFFu, merged);
             if (lane == 0 && merged) atomicAdd(&T.lead->c_merged, merged);
-        } else if (gtid == 0) {
-            // every occurrence of the pair itself goes
+        } else if (rank == WM_CLUSTER - 1 && tid == WM_THREADS - 1) {
+            // every occurrence of the pair itself goes (a thread that seldom has an occurrence: this is a chain of round trips of its own)
             wt_update(A, T, pair, count, false, tau);
         }
         __syncwarp();
@@ -797,18 +798,19 @@ k_word_merges(WordArgs A, uint32_t target) {
                 const uint32_t l = tail_at(tail, i);
                 if (tail_match(tail, l, tail_at(tail, i + 1u))) tail_src[i] = (l & WORD_START_BIT) | fresh;
             }
-            tail_pairs(A, T, older, stale, gtid, true, tau, dst + kept_all);
-            if (gtid == 0) {
-                if (stale) {      // the last copied symbol and the first older one
+            tail_pairs(A, T, older, stale, gtid_mid, true, tau, dst + kept_all);
+            // single updates, each a chain of round trips, by threads of different SMs
+            if (tid == WM_THREADS - 1) {
+                if (rank == 0 && stale) {      // the last copied symbol and the first older one
                     uint32_t i = tail.limit - 1u, l = tail_at(tail, i);
-                    while (i > 0u && tail_match(tail, tail_at(tail, i - 1u), l)) l = tail_at(tail, --i);
-                    if (tail_match(tail, l, tail_at(tail, i + 1u))) l = fresh;
-                    const uint32_t r = __ldcg(older);
+                    const uint32_t behind = tail_at(tail, i + 1u), r = __ldcg(older);
+                    uint32_t prev = i > 0u ? tail_at(tail, i - 1u) : WORD_START_BIT, next = behind;
+                    while (i > 0u && tail_match(tail, prev, l)) { next = l; l = prev; i--; prev = i > 0u ? tail_at(tail, i - 1u) : WORD_START_BIT; }
+                    if (tail_match(tail, l, next)) l = fresh;
                     if (tail_counted(l, r)) tail_pair(A, T, l, r, true, tau);
                 }
-                if (dropped) {    // the front's occurrences of the pair itself go (the tail's went one by one)
+                if (rank == 1 && dropped)      // the front's occurrences of the pair itself go (the tail's went one by one)
                     wt_update(A, T, pair, dropped, false, tau);
-                }
             }
             __syncwarp();
         }
