@@ -6,7 +6,8 @@
 // the left symbol, pair), and the merge that takes (x, y) reads the list of max(x, y) and keeps the entries of its own pair.
 // Byte pairs have exact lists of their own (k_dict_lists).  And a pair's count never rises after the merge that made it, so the
 // arg-max needs only the pairs above a threshold: a candidate list made by a scan of the pair table, to which a merge adds the
-// new pairs that reach the threshold; when the best candidate falls below it, the table is scanned again.
+// new pairs that reach the threshold; when the best candidate falls below it, the table is scanned again.  ("literal" runs, whose text's
+// tail is kept by itself, can raise a count again: a rise across the threshold makes a candidate whenever it happens.)
 //
 // What bounds a merge is then a chain of dependent memory round trips (occurrence list -> records -> pair table -> candidates'
 // counts), and the barriers between its two phases, not bandwidth.  So the loop runs inside ONE thread-block cluster: 16 CTAs on

@@ -5,8 +5,8 @@ UTF-8 bytes become one token each, then the merge rules of the trained model are
 order they were learned, each over the whole token list, left to right.  The result object has the
 reference's fields {tokens, text, vocab, vocabStrings}; without a model the call raises the
 reference's 'No trained model available', and a model without merges gives the bytes back.
-The passes run in libb200bpe.so (b200bpe_replay_*): rounds of "smallest rule rank present" +
-single-pass scan and compaction.
+The passes run in libb200bpe.so (b200bpe_replay_*): the text falls apart into segments that no rule crosses, each
+encoded by itself, smallest rule rank first; texts with very long segments take rounds over the whole list.
 """
 from __future__ import annotations
 
