@@ -57,7 +57,7 @@ struct WordArgs {
     const uint32_t* weight;
     const uint32_t* byte_list;        // occurrences of the byte pairs
     const uint32_t* byte_off;
-    uint2* entries;                   // {position of the left symbol, left << 16 | right}
+    uint2* entries;                   // {position of the left symbol, left << 16 | right}, room for 2 * positions
     uint2* segment;                   // [symbol] = {first entry, end}
     uint32_t* usual;                  // [symbol] = positions it usually covers (always, but for symbols made of a run of equal ones)
     uint32_t positions;               // rec[positions] begins a word, and nothing lies behind it
@@ -77,7 +77,7 @@ struct WordShared {
     uint32_t xflags[WM_CLUSTER];
     unsigned long long wbest[WM_THREADS / 32];
     uint32_t queued, ncand, flags, inserted;
-    uint32_t c_entries, c_inserted, c_merged;   // the cluster's counters: those of CTA 0 are the ones in use
+    uint32_t c_entries, c_inserted, c_merged, c_spilled;   // the cluster's counters: those of CTA 0 are the ones in use
     uint32_t kept[WM_CLUSTER * WM_THREADS / 32];          // tail symbols that every warp of the cluster copies
     uint32_t tail_queue[4096], tail_queued;               // matches in this CTA's part of the tail
     WordState init;
@@ -583,7 +583,7 @@ k_word_merges(WordArgs A, uint32_t target) {
     __syncthreads();
     if (tid == 0) {
         s.queued = 0u; s.flags = 0u; s.inserted = 0u; s.ncand = s.init.tau == ~0ull ? 0u : nc;
-        s.c_entries = s.init.entries; s.c_inserted = 0u; s.c_merged = 0u; s.tail_queued = 0u;
+        s.c_entries = s.init.entries; s.c_inserted = 0u; s.c_merged = 0u; s.c_spilled = 0u; s.tail_queued = 0u;
     }
     cluster_barrier();           // also: everybody has read the control block before anybody writes it
     uint32_t done = s.init.merges_done, next_id = s.init.next_id, symbols = s.init.symbols, scans = s.init.scans;
@@ -595,6 +595,8 @@ k_word_merges(WordArgs A, uint32_t target) {
     const uint32_t occ_start = s.init.occupied;
     const uint32_t room = (1u << A.table_log2) / 4u * 3u;
     uint32_t flags = 0u;
+    uint32_t spilled_before = 0u;            // c_spilled after the merge before
+    uint2* const spill_end = A.entries + 2u * (size_t)A.positions;
     if (early || status) return;             // the same in every CTA
 
     while (done < target) {
@@ -694,8 +696,7 @@ k_word_merges(WordArgs A, uint32_t target) {
             if (right) A.entries[at] = make_uint2(p, k3);
         };
         // Phase 2 of one occurrence.
-        auto rewrite = [&](uint32_t qi) {
-            const uint2 o = s.queue[qi];
+        auto rewrite = [&](uint2 o) {
             if (o.x == ~0u) return;
             const uint32_t p = o.x, span = o.y & 0x7FFFu, e = p + span - 1u;
             const uint32_t rp = A.rec[p];
@@ -706,16 +707,37 @@ k_word_merges(WordArgs A, uint32_t target) {
                 for (uint32_t q = p + wp_span(rp); q <= e;) {
                     const uint32_t rq = A.rec[q];
                     A.rec[q] = 0u;
-                    q += wp_span(rq);
+                    q += max(wp_span(rq), 1u);
                 }
             }
             A.rec[e] = span << 16;
             A.rec[p] = fresh | span << 16 | (rp & WP_START);
         };
-        // The list in rounds of WM_UNROLL entries per thread; `f` takes the queued occurrences whenever the queue could overflow, and
-        // at the end.  Returns whether the queue was emptied before the end.
-        auto walk = [&](auto&& f) -> bool {
-            bool spilled = false;
+        // The queue's first n occurrences, with what phase 1 found out about them, to the end of the entries' buffer, downwards.  Phase 2 takes
+        // them from there and looks at no neighbour again: in a run of equal symbols the neighbours are another thread's to rewrite, and
+        // may be gone.  There is room: an occurrence writes two entries at most and ends a position, so with L symbols left after
+        // this merge the lists hold 2 (positions - L) entries at most; and every occurrence leaves a symbol, so L are spilled at most.
+        auto spill = [&](uint32_t n) {
+            uint32_t mine = 0u;
+            for (uint32_t i0 = 0; i0 < n; i0 += WM_THREADS) {
+                const uint32_t i = i0 + tid;                 // (the thread that has looked at it)
+                mine += __popc(__ballot_sync(0xFFFFFFFFu, i < n && s.queue[i].x != ~0u));
+            }
+            uint32_t at = 0u;
+            if (lane == 0 && mine) at = atomicAdd(&T.lead->c_spilled, mine) - spilled_before;
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            for (uint32_t i0 = 0; i0 < n; i0 += WM_THREADS) {
+                const uint32_t i = i0 + tid;
+                const uint2 o = i < n ? s.queue[i] : make_uint2(~0u, 0u);
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, o.x != ~0u);
+                if (o.x != ~0u) *(spill_end - 1u - (at + __popc(m & ((1u << lane) - 1u)))) = o;
+                at += __popc(m);
+            }
+        };
+        // The list in rounds of WM_UNROLL entries per thread; the queued occurrences are taken whenever the queue could overflow
+        // (only a list of more than one round can), and at the end.
+        const bool spills = len > STEP * WM_UNROLL;          // the same in every CTA
+        auto walk = [&]() {
             for (uint32_t base = 0; base < len; base += STEP * WM_UNROLL) {
                 uint32_t pos[WM_UNROLL];
                 bool hit[WM_UNROLL];
@@ -744,16 +766,16 @@ k_word_merges(WordArgs A, uint32_t target) {
                 const bool last = base + STEP * WM_UNROLL >= len;
                 if (!last) __syncthreads();          // everybody has read the fill before the next round adds to it
                 if (last || n + WM_THREADS * WM_UNROLL > WM_QUEUE) {
-                    for (uint32_t i = tid; i < n; i += WM_THREADS) f(i);
+                    for (uint32_t i = tid; i < n; i += WM_THREADS) apply(i);
+                    __syncwarp();
                     if (!last) {
-                        spilled = true;
+                        spill(n);
                         __syncthreads();
                         if (tid == 0) s.queued = 0u;
                         __syncthreads();
                     }
                 }
             }
-            return spilled;
         };
         static_assert(WM_THREADS * WM_UNROLL <= WM_QUEUE, "a round fits the queue");
         if (LITERAL) {
@@ -761,7 +783,7 @@ k_word_merges(WordArgs A, uint32_t target) {
             if (lane < WM_CLUSTER) cluster.map_shared_rank(&s, lane)->kept[(tid >> 5) * WM_CLUSTER + rank] = kept;
             __syncthreads();
         }
-        const bool spilled = walk(apply);
+        walk();
         if (LITERAL) {
             // the tail's matches from the last thread down: where both are few, other warps than those with the dictionary's occurrences
             for (uint32_t i = WM_THREADS - 1u - tid; i < min(s.tail_queued, TAIL_QUEUE); i += WM_THREADS) tail_match_changes(A, T, tail, s.tail_queue[i], tau);
@@ -816,31 +838,14 @@ k_word_merges(WordArgs A, uint32_t target) {
             __syncwarp();
         }
         // ── phase 2: the records; the next merge's pair ──
-        if (!spilled) {
+        {
             const uint32_t n = s.queued;
-            for (uint32_t i = tid; i < n; i += WM_THREADS) rewrite(i);
-        } else {
-            // the queue did not hold everything: find the occurrences again (their own records are as they were in phase 1: nobody
-            // else rewrites them, and the left neighbour of a run is not part of this merge)
-            __syncthreads();
-            if (tid == 0) s.queued = 0u;
-            __syncthreads();
-            walk([&](uint32_t qi) {
-                const uint32_t p = s.queue[qi].x;
-                const uint32_t rp = A.rec[p];
-                bool ok = wp_sym(rp) == a;
-                const uint32_t la = wp_span(rp), q = p + la;
-                const uint32_t rq = ok ? A.rec[q] : WP_START;
-                ok = ok && !(rq & WP_START) && wp_sym(rq) == b;
-                uint32_t r = q + wp_span(rq);
-                if (a == b && ok) {
-                    if (!(rp & WP_START) && wp_sym(A.rec[p - wp_span(A.rec[p - 1])]) == a) ok = false;
-                    uint32_t rr = A.rec[r];
-                    while (ok && !(rr & WP_START) && wp_sym(rr) == a) { r += wp_span(rr); rr = A.rec[r]; }
-                }
-                s.queue[qi] = ok ? make_uint2(p, (r - p) | (a == b ? 0u : la << 16)) : make_uint2(~0u, 0u);
-                rewrite(qi);
-            });
+            for (uint32_t i = tid; i < n; i += WM_THREADS) rewrite(s.queue[i]);
+        }
+        if (spills) {
+            const uint32_t all = T.lead->c_spilled, n = all - spilled_before;     // (nobody spills before the next cluster barrier)
+            for (uint32_t i = gtid; i < n; i += STEP) rewrite(__ldcg(spill_end - 1 - i));
+            spilled_before = all;
         }
         if (gtid == 0) {
             const uint32_t e1 = s.c_entries;
