@@ -713,6 +713,19 @@ __global__ void k_doc_token_offsets(const uint64_t* __restrict__ chunk_base, con
         tok_offsets[d] = chunk_offsets[chunk_base[d]];
 }
 
+// Lets a kernel be launched with as much dynamic shared memory as a CTA can have.  The limit is a setting of the kernel, which every
+// handle shares: set to what one trie needs, it would refuse the launches of a handle with a larger one.
+template <class Kernel>
+static cudaError_t allow_all_shared_memory(Kernel* kernel) {
+    int device = 0, most = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+    return e;
+}
+
 struct Tokenizer {
     Ctx* ctx = nullptr;
     uint32_t node_count = 0, edge_count = 0, max_token_len = 0, chunk = 0;
@@ -841,13 +854,13 @@ struct Tokenizer {
         else if (ck_d == 2) f(integral_constant<int, 2>{}, integral_constant<int, 512>{});
         else f(integral_constant<int, 3>{}, integral_constant<int, 512>{});
     }
-    // The shared memory that the split walk of this trie asks for (at creation: later launches find the kernel loaded).
+    // (At creation: later launches find the kernel loaded.)
     cudaError_t prepare_split() const {
         cudaError_t e = cudaSuccess;
         if ((ck_d == 0 && !hybrid) || walk_smem() + sizeof(SplitShared<512>) > 227u * 1024) return e;
         for_split([&](auto d, auto threads) {
             constexpr int D = decltype(d)::value, T = decltype(threads)::value;
-            e = cudaFuncSetAttribute(k_trie_split<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(walk_smem() + sizeof(SplitShared<T>)));
+            e = allow_all_shared_memory(k_trie_split<D, T>);
         });
         return e;
     }
@@ -1296,22 +1309,15 @@ b200bpe_status b200bpe_tokenizer_create_ex(b200bpe_ctx* c, const void* trie, siz
         B2_TRY(cudaMemcpyAsync(t->d_hot, hot.data(), hot.size() * 4, cudaMemcpyHostToDevice, s));
         B2_TRY(cudaMalloc(&t->d_cold, cold.size() * 8));
         B2_TRY(cudaMemcpyAsync(t->d_cold, cold.data(), cold.size() * 8, cudaMemcpyHostToDevice, s));
-        B2_TRY(cudaFuncSetAttribute(k_trie_walk_hybrid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HY_SMEM_BYTES));
+        B2_TRY(allow_all_shared_memory(k_trie_walk_hybrid));
     } else if (ck_d == 0) {
         B2_TRY(cudaMalloc(&t->d_trans, trans.size() * 8));
         B2_TRY(cudaMemcpyAsync(t->d_trans, trans.data(), trans.size() * 8, cudaMemcpyHostToDevice, s));
-        B2_TRY(cudaFuncSetAttribute(k_trie_walk<TW_THREADS, TW_CACHE_LOG2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    TW_SMEM_BYTES));
+        B2_TRY((allow_all_shared_memory(k_trie_walk<TW_THREADS, TW_CACHE_LOG2, 0>)));
     } else {
         B2_TRY(cudaMalloc(&t->d_cuckoo, cuckoo.size() * 4));
         B2_TRY(cudaMemcpyAsync(t->d_cuckoo, cuckoo.data(), cuckoo.size() * 4, cudaMemcpyHostToDevice, s));
-        if (ck_d == 2) {
-            B2_TRY(cudaFuncSetAttribute(k_trie_walk<CK_THREADS, 0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(cuckoo.size() * 4)));
-        } else {
-            B2_TRY(cudaFuncSetAttribute(k_trie_walk<CK_THREADS, 0, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(cuckoo.size() * 4)));
-        }
+        B2_TRY(ck_d == 2 ? allow_all_shared_memory(k_trie_walk<CK_THREADS, 0, 2>) : allow_all_shared_memory(k_trie_walk<CK_THREADS, 0, 3>));
     }
     B2_TRY(t->prepare_split());
     B2_TRY(cudaMallocHost(&t->h_total, 16 + Tokenizer::SMALL_TOKENS * 4));

@@ -72,3 +72,27 @@ def test_both_sides_of_the_rule(engine, layout, n):
     whole, sliced = (TrieTokenizer(engine, trie, RUNS, {"layout": layout, **o}) for o in ({}, {"encodeSliceBytes": 1 << 20}))
     assert np.array_equal(whole.encodeBytes(data), sliced.encodeBytes(data))
     whole.destroy(), sliced.destroy()
+
+
+@pytest.mark.parametrize("layout", ["auto", "hybrid"])
+def test_a_small_vocabulary_beside_a_large_one(engine, layout):
+    """Handles whose tries ask for different amounts of shared memory, in every order of creation and use."""
+    import torch
+    data, _, sym = small_text(2, 23, 300_000)
+    entries = list(BYTES)
+    for a, b, _, _ in O.train(sym, 8000, "fixed", threads=8)["merges"].tolist():
+        entries.append(entries[a] + entries[b])
+    sizes = [8256, 320, 4096, 600, 2048]
+    toks = [TrieTokenizer.fromVocab(engine, entries[:n], {"layout": layout}) for n in sizes]
+    assert layout == "hybrid" or len({t.deviceLayout for t in toks if t.deviceLayout[0] == 2}) > 1
+    large = np.tile(data, 200)               # beyond the split walk's range: the walk of whole chunks
+    d_text, d_out = torch.from_numpy(data).cuda(), torch.empty(data.size, dtype=torch.int32, device="cuda")
+    for t, n in 2 * list(zip(toks, sizes)):
+        trie = compileVocabToTrie(entries[:n])
+        want = O.encode(data, trie, t.chunkSize)
+        assert np.array_equal(t.encodeBytes(data), want), n
+        k = t.encodeDeviceNoAlloc(d_text.data_ptr(), data.size, d_out.data_ptr(), data.size)
+        assert np.array_equal(d_out[:k].cpu().numpy().astype(np.uint32), want), n
+        assert t.encodeBytes(large).size == O.encode(large, trie, t.chunkSize).size, n
+    for t in toks:
+        t.destroy()
