@@ -99,6 +99,7 @@ SIGNATURES = {
     "b200bpe_tokenizer_last_ms": (C.c_int32, [C.c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "b200bpe_tokenizer_destroy": (None, [C.c_void_p]),
     "b200bpe_decoder_create": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.POINTER(C.c_void_p)]),
+    "b200bpe_decoder_decode": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64, u64p]),
     "b200bpe_decoder_run": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_uint64, u64p]),
     "b200bpe_decoder_read": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_uint64]),
     "b200bpe_decoder_destroy": (None, [C.c_void_p]),

@@ -34,19 +34,22 @@ struct Ctx {
     int rank = 0, world = 1;
     NcclApi nccl;
     void* comm = nullptr;
-    // Device memory of this context's short-lived objects, in the order of its stream: an allocation is a few microseconds when
+    // Device memory of this context's short-lived objects, in the order of a stream (its own, or that of an object with one): an allocation is a few microseconds when
     // the pool has the block, against hundreds for cudaMalloc.  At most POOL_KEEP bytes stay with the pool between calls; the
     // rest goes back to the device at the next synchronisation, and all of it with the context.
     cudaMemPool_t pool = nullptr;
     static constexpr unsigned long long POOL_KEEP = 2ull << 30;
     template <class T>
-    cudaError_t alloc(T** p, size_t bytes) {
+    cudaError_t alloc(T** p, size_t bytes, cudaStream_t on) {
         void* v = nullptr;
-        const cudaError_t e = cudaMallocFromPoolAsync(&v, bytes ? bytes : 1, pool, stream);
+        const cudaError_t e = cudaMallocFromPoolAsync(&v, bytes ? bytes : 1, pool, on);
         *p = static_cast<T*>(v);
         return e;
     }
-    void free(void* p) { if (p) cudaFreeAsync(p, stream); }
+    template <class T>
+    cudaError_t alloc(T** p, size_t bytes) { return alloc(p, bytes, stream); }
+    void free(void* p, cudaStream_t on) { if (p) cudaFreeAsync(p, on); }
+    void free(void* p) { free(p, stream); }
     // Pinned host memory of this context's short-lived objects: cudaMallocHost takes 3 to 5 ms, half of a training call on a page of
     // text.  A few blocks are kept between objects, PINNED_KEEP bytes at most, and go with the context.  A block is only given back when no
     // copy to or from it is on its way.

@@ -5,8 +5,12 @@
 // scan, look-back over the tiles), k_decode_copy copies them.  Both are bound by the gathers from the vocabulary, which L2 holds; at
 // the sizes of a call that is little against the two copies over the bus.
 // 85,000 tokens of a 32,256-entry vocabulary from and to host memory: 7.86 ms token by token on the host, 0.147 ms here.
+//
+// Detokenising is what a server's worker threads do at any time, so a handle does not change once it is made: what a call needs belongs
+// to the call, and the work goes through a stream of the handle's own, apart from a graph that the context's stream may be recording.
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -70,11 +74,11 @@ k_decode_places(const uint32_t* __restrict__ tokens, uint64_t n, const uint64_t*
         }
     }
 }
-// Copies every token's bytes to its place, if all of them fit `cap`.
+// Copies every token's bytes to its place, if all of them fit `cap` (and every tile learned its place).
 __global__ void __launch_bounds__(DC_THREADS)
 k_decode_copy(const uint32_t* __restrict__ tokens, uint64_t n, const uint64_t* __restrict__ off, const uint8_t* __restrict__ bytes, uint32_t entries,
               const uint64_t* __restrict__ place, const unsigned long long* __restrict__ ctl, uint8_t* __restrict__ out, uint64_t cap) {
-    if (ctl[0] > cap) return;
+    if (ctl[0] > cap || (ctl[1] >> 32) != 0ull) return;
     for (uint64_t i = (uint64_t)blockIdx.x * DC_THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * DC_THREADS) {
         const uint32_t t = min(tokens[i], entries);
         const uint64_t from = off[t], len = off[t + 1] - from, to = place[i];
@@ -84,38 +88,46 @@ k_decode_copy(const uint32_t* __restrict__ tokens, uint64_t n, const uint64_t* _
 
 struct Decoder {
     Ctx* ctx = nullptr;
+    cudaStream_t stream = nullptr;
     uint32_t entries = 0;
     uint64_t* d_off = nullptr;
     uint8_t* d_bytes = nullptr;
-    uint64_t* h_ctl = nullptr;      // pinned
-    // the last text, in the context's pool
-    uint8_t* d_out = nullptr;
-    uint64_t n_out = 0;
+    // the text of the last b200bpe_decoder_run
+    std::mutex mutex;
+    uint8_t* d_text = nullptr;
+    uint64_t n_text = 0;
 
     ~Decoder() {
-        if (ctx) {
-            cudaSetDevice(ctx->device);
-            for (void* p : {(void*)d_off, (void*)d_bytes, (void*)d_out}) ctx->free(p);
+        if (!ctx) return;
+        cudaSetDevice(ctx->device);
+        for (void* p : {(void*)d_off, (void*)d_bytes, (void*)d_text}) ctx->free(p, stream);
+        if (stream) {
+            cudaStreamSynchronize(stream);
+            cudaStreamDestroy(stream);
         }
-        if (h_ctl) cudaFreeHost(h_ctl);
     }
 
-    b200bpe_status run(const uint32_t* tokens, uint64_t n) {
-        cudaStream_t s = ctx->stream;
-        ctx->free(d_out);
-        d_out = nullptr;
-        n_out = 0;
+    // Host tokens to bytes on the device: *text, the caller's to free (null without bytes), and their number.
+    b200bpe_status run(const uint32_t* tokens, uint64_t n, uint8_t** text, uint64_t* n_bytes) {
+        cudaStream_t s = stream;
+        *text = nullptr;
+        *n_bytes = 0;
         if (n == 0) return B200BPE_OK;
         const uint64_t tiles = (n + DC_TILE - 1) / DC_TILE;
         uint32_t* d_tok = nullptr;
         uint64_t* place = nullptr;
         unsigned long long* ctl = nullptr;
+        uint8_t* d_out = nullptr;
+        void* pinned = nullptr;
+        size_t pinned_bytes = 16;
         uint64_t cap = n * 8;       // a guess; an output that needs more is copied again
         auto work = [&]() -> b200bpe_status {
-            B2_CUDA(ctx->alloc(&d_tok, n * 4));
-            B2_CUDA(ctx->alloc(&place, n * 8));
-            B2_CUDA(ctx->alloc(&ctl, (tiles + 2) * 8));
-            B2_CUDA(ctx->alloc(&d_out, cap));
+            B2_CUDA(ctx->alloc_pinned(&pinned, &pinned_bytes));
+            uint64_t* h_ctl = static_cast<uint64_t*>(pinned);
+            B2_CUDA(ctx->alloc(&d_tok, n * 4, s));
+            B2_CUDA(ctx->alloc(&place, n * 8, s));
+            B2_CUDA(ctx->alloc(&ctl, (tiles + 2) * 8, s));
+            B2_CUDA(ctx->alloc(&d_out, cap, s));
             B2_CUDA(cudaMemcpyAsync(d_tok, tokens, n * 4, cudaMemcpyHostToDevice, s));
             B2_CUDA(cudaMemsetAsync(ctl, 0, (tiles + 2) * 8, s));
             const int most = ctx->sm_count * 8;
@@ -127,19 +139,33 @@ struct Decoder {
             B2_CUDA(cudaStreamSynchronize(s));
             if ((uint32_t)(h_ctl[1] >> 32) != 0u) return B200BPE_ERR_LOOKBACK_TIMEOUT;
             if (h_ctl[0] > cap) {
-                ctx->free(d_out);
+                ctx->free(d_out, s);
                 d_out = nullptr;
                 cap = h_ctl[0];
-                B2_CUDA(ctx->alloc(&d_out, cap));
+                B2_CUDA(ctx->alloc(&d_out, cap, s));
                 k_decode_copy<<<grid, DC_THREADS, 0, s>>>(d_tok, n, d_off, d_bytes, entries, place, ctl, d_out, cap);
                 B2_CUDA(cudaGetLastError());
             }
-            n_out = h_ctl[0];
+            *text = d_out;
+            *n_bytes = h_ctl[0];
+            d_out = nullptr;
             return B200BPE_OK;
         };
         const b200bpe_status r = work();
-        for (void* p : {(void*)d_tok, (void*)place, (void*)ctl}) ctx->free(p);
+        if (r != B200BPE_OK) {
+            cudaGetLastError();              // (an allocation that failed is nobody else's error)
+            cudaStreamSynchronize(s);        // nothing is on its way to the pinned block
+        }
+        for (void* p : {(void*)d_tok, (void*)place, (void*)ctl, (void*)d_out}) ctx->free(p, s);
+        ctx->free_pinned(pinned, pinned_bytes);
         return r;
+    }
+
+    b200bpe_status read(const uint8_t* text, uint8_t* out, uint64_t n) {
+        if (n == 0) return B200BPE_OK;
+        B2_CUDA(cudaMemcpyAsync(out, text, n, cudaMemcpyDeviceToHost, stream));
+        B2_CUDA(cudaStreamSynchronize(stream));
+        return B200BPE_OK;
     }
 };
 
@@ -161,12 +187,12 @@ b200bpe_status b200bpe_decoder_create(b200bpe_ctx* c, const uint8_t* bytes, cons
     Decoder& d = h->d;
     d.ctx = &c->c;
     d.entries = n_entries;
-    cudaStream_t s = c->c.stream;
     static const uint8_t replacement[3] = {0xEF, 0xBF, 0xBD};
     const uint64_t end = n + 3;
-    cudaError_t e = c->c.alloc(&d.d_off, ((uint64_t)n_entries + 2) * 8);
-    if (e == cudaSuccess) e = c->c.alloc(&d.d_bytes, end);
-    if (e == cudaSuccess) e = cudaMallocHost(&d.h_ctl, 16);
+    cudaError_t e = cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking);
+    cudaStream_t s = d.stream;
+    if (e == cudaSuccess) e = c->c.alloc(&d.d_off, ((uint64_t)n_entries + 2) * 8, s);
+    if (e == cudaSuccess) e = c->c.alloc(&d.d_bytes, end, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d.d_off, offsets, ((uint64_t)n_entries + 1) * 8, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d.d_off + n_entries + 1, &end, 8, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && n) e = cudaMemcpyAsync(d.d_bytes, bytes, n, cudaMemcpyHostToDevice, s);
@@ -177,23 +203,36 @@ b200bpe_status b200bpe_decoder_create(b200bpe_ctx* c, const uint8_t* bytes, cons
     return B200BPE_OK;
 }
 
+b200bpe_status b200bpe_decoder_decode(b200bpe_decoder* h, const uint32_t* tokens, uint64_t n, uint8_t* out, uint64_t cap, uint64_t* n_bytes_out) {
+    if (!h || (!tokens && n) || (!out && cap) || !n_bytes_out) return B200BPE_ERR_BAD_ARG;
+    Decoder& d = h->d;
+    B2_CUDA(cudaSetDevice(d.ctx->device));
+    uint8_t* text = nullptr;
+    b200bpe_status r = d.run(tokens, n, &text, n_bytes_out);
+    if (r == B200BPE_OK) r = *n_bytes_out > cap ? B200BPE_ERR_CAPACITY : d.read(text, out, *n_bytes_out);
+    d.ctx->free(text, d.stream);
+    return r;
+}
+
 b200bpe_status b200bpe_decoder_run(b200bpe_decoder* h, const uint32_t* tokens, uint64_t n, uint64_t* n_bytes_out) {
     if (!h || (!tokens && n) || !n_bytes_out) return B200BPE_ERR_BAD_ARG;
-    *n_bytes_out = 0;
-    B2_CUDA(cudaSetDevice(h->d.ctx->device));
-    const b200bpe_status r = h->d.run(tokens, n);
-    if (r == B200BPE_OK) *n_bytes_out = h->d.n_out;
+    Decoder& d = h->d;
+    B2_CUDA(cudaSetDevice(d.ctx->device));
+    std::lock_guard<std::mutex> lock(d.mutex);
+    d.ctx->free(d.d_text, d.stream);
+    const b200bpe_status r = d.run(tokens, n, &d.d_text, &d.n_text);
+    *n_bytes_out = d.n_text;
     return r;
 }
 
 b200bpe_status b200bpe_decoder_read(b200bpe_decoder* h, uint8_t* out, uint64_t cap) {
-    if (!h || (!out && h->d.n_out)) return B200BPE_ERR_BAD_ARG;
-    if (cap < h->d.n_out) return B200BPE_ERR_CAPACITY;
-    if (h->d.n_out == 0) return B200BPE_OK;
-    B2_CUDA(cudaSetDevice(h->d.ctx->device));
-    B2_CUDA(cudaMemcpyAsync(out, h->d.d_out, h->d.n_out, cudaMemcpyDeviceToHost, h->d.ctx->stream));
-    B2_CUDA(cudaStreamSynchronize(h->d.ctx->stream));
-    return B200BPE_OK;
+    if (!h) return B200BPE_ERR_BAD_ARG;
+    Decoder& d = h->d;
+    std::lock_guard<std::mutex> lock(d.mutex);
+    if (!out && d.n_text) return B200BPE_ERR_BAD_ARG;
+    if (cap < d.n_text) return B200BPE_ERR_CAPACITY;
+    B2_CUDA(cudaSetDevice(d.ctx->device));
+    return d.read(d.d_text, out, d.n_text);
 }
 
 void b200bpe_decoder_destroy(b200bpe_decoder* h) { delete h; }

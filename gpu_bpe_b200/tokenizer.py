@@ -8,6 +8,7 @@ addition: many documents per call, each encoded as its own encodeBytes call woul
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 
@@ -15,6 +16,9 @@ from . import _lib
 from .trie import compileVocabToTrie, parseHeader
 
 UTF8_REPLACEMENT = [0xEF, 0xBF, 0xBD]  # tokenizer.js:18
+# Tokens from which decode goes to the device (vocabulary of 32,256): the loop takes 18, 81 and 159 us for 100, 500 and 1,000 tokens, the
+# device, whose copies and waits are the same for any, 67, 70 and 73 us.
+DECODE_ON_DEVICE = 512
 
 
 class TrieTokenizer:
@@ -23,6 +27,7 @@ class TrieTokenizer:
         self._engine = engine
         self._vocab = vocab if vocab is not None else [[i] for i in range(256)]
         self._dh = self._decode_entries = None
+        self._decode_lock = threading.Lock()     # round the decoder's handle: threads may decode at any time
         header = parseHeader(trieData)   # raises the reference's errors for bad magic / version / length
         buf = np.frombuffer(trieData, np.uint8)
         h = C.c_void_p()
@@ -128,14 +133,24 @@ class TrieTokenizer:
             _lib.lib().b200bpe_decoder_destroy(self._dh)
         self._dh = self._decode_entries = None
 
-    def decode(self, tokens) -> bytes:
-        if isinstance(tokens, np.ndarray) and tokens.dtype == np.uint32 and tokens.ndim == 1 and tokens.size and self._decoder() is not None:
+    def _decode_on_device(self, tokens) -> bytes | None:
+        with self._decode_lock:
+            if self._decoder() is None:
+                return None
             t = np.ascontiguousarray(tokens)
-            n = C.c_uint64()
-            if _lib.lib().b200bpe_decoder_run(self._dh, t.ctypes.data, t.size, C.byref(n)) == 0:
+            text, n = np.empty(8 * t.size, np.uint8), C.c_uint64()      # (a guess)
+            for _ in range(2):
+                st = _lib.lib().b200bpe_decoder_decode(self._dh, t.ctypes.data, t.size, text.ctypes.data, text.size, C.byref(n))
+                if _lib.STATUS[st] != "CAPACITY":
+                    break
                 text = np.empty(n.value, np.uint8)
-                _lib.check(_lib.lib().b200bpe_decoder_read(self._dh, text.ctypes.data, text.size), "b200bpe_decoder_read")
-                return text.tobytes()
+            return text[:n.value].tobytes() if st == 0 else None
+
+    def decode(self, tokens) -> bytes:
+        if isinstance(tokens, np.ndarray) and tokens.dtype == np.uint32 and tokens.ndim == 1 and tokens.size >= DECODE_ON_DEVICE:
+            text = self._decode_on_device(tokens)
+            if text is not None:
+                return text
         out = bytearray()
         for t in tokens:
             t = int(t)
@@ -143,8 +158,9 @@ class TrieTokenizer:
         return bytes(out)
 
     def destroy(self):
-        if self._engine._ctx is not None:
-            self._drop_decoder()
+        with self._decode_lock:
+            if self._engine._ctx is not None:
+                self._drop_decoder()
         if self._h is not None:
             _lib.lib().b200bpe_tokenizer_destroy(self._h)
             self._h = None

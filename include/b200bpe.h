@@ -243,10 +243,12 @@ b200bpe_status b200bpe_tokenizer_last_ms(b200bpe_tok*, double* walk_ms, double* 
 void b200bpe_tokenizer_destroy(b200bpe_tok*);
 
 /* Token ids back to bytes (TrieTokenizer.decode, src/bpe/tokenizer/tokenizer.js): entry t of the vocabulary is bytes[offsets[t]] up to
- * bytes[offsets[t + 1]]; an id of n_entries or more gives U+FFFD.  _run decodes host tokens into a device buffer of the handle and says how
- * many bytes that made, _read copies them to the host.  One call at a time per handle. */
+ * bytes[offsets[t + 1]]; an id of n_entries or more gives U+FFFD.  _decode takes host tokens to host bytes and says how many there are
+ * (CAPACITY: more than cap, none are written); any number of threads can call it on one handle.  In two steps: _run decodes into a device
+ * buffer of the handle and says how many bytes that made, _read copies them to the host; the two belong together, so here one thread at a time. */
 typedef struct b200bpe_decoder b200bpe_decoder;
 b200bpe_status b200bpe_decoder_create(b200bpe_ctx*, const uint8_t* bytes, const uint64_t* offsets, uint32_t n_entries, b200bpe_decoder** out);
+b200bpe_status b200bpe_decoder_decode(b200bpe_decoder*, const uint32_t* tokens, uint64_t n, uint8_t* out, uint64_t cap, uint64_t* n_bytes_out);
 b200bpe_status b200bpe_decoder_run(b200bpe_decoder*, const uint32_t* tokens, uint64_t n, uint64_t* n_bytes_out);
 b200bpe_status b200bpe_decoder_read(b200bpe_decoder*, uint8_t* out, uint64_t cap);
 void b200bpe_decoder_destroy(b200bpe_decoder*);
