@@ -140,7 +140,8 @@ b200bpe_status b200bpe_train(b200bpe_ctx*, const uint8_t* bytes, const uint8_t* 
 /* The same run, split into steps so that a caller can keep the corpus resident on the device,
  * repeat runs, and inspect intermediate state.  create uploads and tags the symbols
  * (trainer.js:62-80,115-121,173-175); create_from_symbols takes already tagged u32 symbols
- * (bit 16 = word start, train.wgsl:36-37); *_device variants take device pointers. */
+ * (bit 16 = word start, train.wgsl:36-37); *_device variants take device pointers, which are read while create and
+ * reset run, and at no other time: in between the caller may overwrite the buffers, and without a reset free them. */
 b200bpe_status b200bpe_trainer_create(b200bpe_ctx*, const uint8_t* bytes, const uint8_t* word_starts, uint64_t n,
                                       const b200bpe_train_opts*, b200bpe_trainer** out);
 b200bpe_status b200bpe_trainer_create_device(b200bpe_ctx*, const uint8_t* d_bytes, const uint8_t* d_word_starts,
