@@ -162,6 +162,7 @@ struct Trainer {
     // timing
     WordPath* words = nullptr;    // training on the distinct words, while by_words
     bool by_words = false;
+    bool words_refused = false;   // the dictionary did not take this text, or could not hold the run: the symbol buffers from now on
     bool classic = false;         // the symbol buffers and all that goes with them are allocated
     cudaEvent_t ev_run0 = nullptr, ev_run1 = nullptr;
     double last_run_ms = 0, last_reset_ms = 0;
@@ -173,6 +174,9 @@ struct Trainer {
     b200bpe_status init_state();
     b200bpe_status init_classic();
     bool words_eligible() const;
+    b200bpe_status init_words();
+    void drop_words();
+    b200bpe_status again_on_symbol_buffers(std::chrono::steady_clock::time_point t0);
     b200bpe_status keep_inputs();
     const uint8_t* src_bytes() const { return kept_bytes ? kept_bytes : d_bytes; }
     const uint8_t* src_mask() const { return !has_mask ? nullptr : kept_mask ? kept_mask : d_mask; }
@@ -288,7 +292,7 @@ b200bpe_status Trainer::alloc_common() {
 // Which runs train on the dictionary of distinct words: those on one GPU, new ids above the byte values, no option that
 // is about the other path's kernels (a recount per merge, the test of its bounded wait).  Positions are 32-bit with a bit to spare.
 bool Trainer::words_eligible() const {
-    return ctx->world == 1 && !(opts.flags & B200BPE_FLAG_FULL_RECOUNT) && !opts.test_first_tile &&
+    return !words_refused && ctx->world == 1 && !(opts.flags & B200BPE_FLAG_FULL_RECOUNT) && !opts.test_first_tile &&
            opts.first_token_id >= 256 && n0 < (1ull << 31);
 }
 
@@ -303,6 +307,55 @@ b200bpe_status Trainer::keep_inputs() {
     return B200BPE_OK;
 }
 
+// The dictionary, if it takes the text and there is memory for it; otherwise everything that belongs to it is given back.
+b200bpe_status Trainer::init_words() {
+    b200bpe_status r = B200BPE_OK;
+    if (!words) {
+        words = new WordPath();
+        r = words->create(ctx, n0, merges_goal, opts.table_log2, opts.compat_mode == B200BPE_COMPAT_LITERAL);
+    }
+    const uint64_t before = words->launches;
+    if (r == B200BPE_OK) r = keep_inputs();
+    if (r == B200BPE_OK) r = words->build(src_bytes(), src_mask(), d_sym_init, opts.first_token_id, &by_words);
+    launches += words->launches - before;
+    if (r == B200BPE_OK && by_words) return r;
+    by_words = false;
+    drop_words();
+    if (own_inputs || r != B200BPE_OK) words_refused = true;    // (a caller's device buffers may hold another text at the next reset)
+    return r == B200BPE_ERR_OOM ? B200BPE_OK : r;
+}
+
+// Gives back what training on the dictionary holds.  The symbol buffers come from cudaMalloc: where memory is short, the pool's goes back first.
+void Trainer::drop_words() {
+    delete words;
+    words = nullptr;
+    for (uint8_t** p : {&kept_bytes, &kept_mask}) { ctx->free(*p); *p = nullptr; }
+    cudaStreamSynchronize(ctx->stream);
+    size_t have = 0, all = 0;
+    if (cudaMemGetInfo(&have, &all) == cudaSuccess && have < 16 * n0) cudaMemPoolTrimTo(ctx->pool, 0);
+    cudaGetLastError();      // (an allocation that failed is no error of the run)
+}
+
+// A run that the dictionary cannot finish, from its start to where it was.
+b200bpe_status Trainer::again_on_symbol_buffers(std::chrono::steady_clock::time_point t0) {
+    const uint32_t had = merges_done;
+    B2_CUDA(cudaStreamSynchronize(ctx->stream));
+    words_refused = own_inputs;
+    by_words = false;
+    early_stop = false;
+    merges_done = 0;
+    cur_n = n0;
+    uint8_t *bytes = kept_bytes, *mask = kept_mask;      // the text has to outlive the dictionary
+    kept_bytes = kept_mask = nullptr;
+    drop_words();
+    kept_bytes = bytes;
+    kept_mask = mask;
+    b200bpe_status r = init_classic();
+    for (uint8_t** p : {&kept_bytes, &kept_mask}) { ctx->free(*p); *p = nullptr; }
+    if (r == B200BPE_OK && had) r = run_classic(had, 0, nullptr, nullptr, nullptr, nullptr, t0);
+    return r;
+}
+
 // Puts everything back to the state of a fresh BPETrainer.train call (trainer.js:187-196), from the resident inputs.
 b200bpe_status Trainer::init_state() {
     cudaStream_t s = ctx->stream;
@@ -315,16 +368,8 @@ b200bpe_status Trainer::init_state() {
     std::memset(&stats, 0, sizeof(stats));
     by_words = false;
     if (words_eligible()) {
-        if (!words) {
-            words = new WordPath();
-            b200bpe_status r = words->create(ctx, n0, merges_goal, opts.table_log2, opts.compat_mode == B200BPE_COMPAT_LITERAL);
-            if (r) return r;
-        }
-        const uint64_t before = words->launches;
-        b200bpe_status r = keep_inputs();
-        if (r == B200BPE_OK) r = words->build(src_bytes(), src_mask(), d_sym_init, opts.first_token_id, &by_words);
+        b200bpe_status r = init_words();
         if (r) return r;
-        launches += words->launches - before;
     }
     if (!by_words) {
         b200bpe_status r = init_classic();
@@ -573,25 +618,18 @@ b200bpe_status Trainer::run_words(uint32_t until, uint32_t start_done, uint32_t*
         const WordState st = w.h_state[i];
         tail++;
         if (st.status & ~(uint32_t)WS_GROW) {
-            B2_CUDA(cudaStreamSynchronize(s));
-            by_words = false;
-            early_stop = false;
-            const uint32_t had = merges_done;
-            if (st.status == WS_TAIL && had == 0 && w.tail_share < WordPath::TAIL_LONG) {
+            if (st.status == WS_TAIL && merges_done == 0 && w.tail_share < WordPath::TAIL_LONG) {
                 // a "literal" run whose tail is too short for its first merges: the same again with a longer one
+                B2_CUDA(cudaStreamSynchronize(s));
                 w.tail_share = WordPath::TAIL_LONG;
                 const uint64_t before = w.launches;
                 b200bpe_status r = w.build(src_bytes(), src_mask(), d_sym_init, opts.first_token_id, &by_words);
-                if (r) return r;
                 launches += w.launches - before;
-                if (by_words) { head = tail = 0; enqueued = 0; continue; }
+                if (r && r != B200BPE_ERR_OOM) return r;
+                if (r == B200BPE_OK && by_words) { head = tail = 0; enqueued = 0; continue; }
             }
-            // a pair table or candidate list that filled up within one merge: run again on the symbol buffers
-            merges_done = 0;
-            cur_n = n0;
-            b200bpe_status r = init_classic();
-            if (r == B200BPE_OK && had) r = run_classic(had, 0, nullptr, nullptr, nullptr, nullptr, t0);
-            return r;
+            // a pair table or candidate list that filled up within one merge, or a merge that reaches past the tail
+            return again_on_symbol_buffers(t0);
         }
         if (timed) {
             float ms = 0;
@@ -623,6 +661,7 @@ b200bpe_status Trainer::run_words(uint32_t until, uint32_t start_done, uint32_t*
         if (st.status == WS_GROW) {
             // the batches behind this one found the same status and did nothing; the next ones start where this one stopped
             b200bpe_status r = w.grow();
+            if (r == B200BPE_ERR_OOM) return again_on_symbol_buffers(t0);
             if (r) return r;
             launches += 2;
             tail = head;
