@@ -396,28 +396,44 @@ def main():
                                      target_vocab_size=256 + n_goal, compat_mode=mode, flags=flags | _lib.FLAG_TIME_KERNELS)
         barrier()
         prof.run()
-        ks = prof.kernel_stats()
+        ks, ws = prof.kernel_stats(), prof.word_stats()
         prof.destroy()
-        kern = {}
-        for name in ("pair_count", "argmax", "merge_compact"):
-            ms_tot, launches, nb = ks[f"{name}_ms"], ks[f"{name}_launches"], ks[f"{name}_bytes"]
-            gbs = (nb / 1e9) / (ms_tot / 1e3) if ms_tot > 0 else 0.0
-            kern[name] = {"ms_total": ms_tot, "launches": launches, "avg_us": 1e3 * ms_tot / max(1, launches),
-                          "algorithmic_GB": nb / 1e9, "achieved_GBps": gbs, "frac_of_peak": gbs / peak}
-        kern["pair_count"]["skipped_launches"] = ks["pair_count_skipped_launches"]
-        kern["pair_count"]["skipped_ms_total"] = ks["pair_count_skipped_ms"]
-        if world > 1:
-            kern["exchange"] = {"ms_total": ks["exchange_ms"], "launches": ks["exchange_launches"],
-                                "avg_us": 1e3 * ks["exchange_ms"] / max(1, ks["exchange_launches"]), "kind": exchange}
-        dom = max(("pair_count", "argmax", "merge_compact"), key=lambda k: kern[k]["ms_total"])
-        roofline = {"bound": "hbm", "kernel": "k_" + dom, "achieved": kern[dom]["achieved_GBps"], "peak": peak, "unit": "GB/s",
-                    "frac": kern[dom]["frac_of_peak"], "peak_source": peak_src,
-                    "traffic": NCU_DRAM_PER_ALGORITHMIC_BYTE[dom] * kern[dom]["algorithmic_GB"] * 1e9 / max(1, kern[dom]["launches"]),
-                    "traffic_how": "DRAM read + write bytes per launch: the ncu ratio of DRAM to algorithmic bytes for this kernel "
-                                   "(one capture, summary under profiles/) x the algorithmic bytes of an average launch",
-                    "per_launch_algorithmic_bytes": kern[dom]["algorithmic_GB"] * 1e9 / max(1, kern[dom]["launches"]),
-                    "avg_launch_us": kern[dom]["avg_us"], "kernels": kern,
-                    "how": "one extra run with CUDA events around every kernel on the library's stream (no graph), this rank"}
+        if ws["launches"]:
+            # training on the dictionary of distinct words: one kernel, a whole batch of merges per launch
+            gbs = ws["bytes"] / 1e9 / (ws["merge_ms"] / 1e3) if ws["merge_ms"] > 0 else 0.0
+            kern = {"word_merges": {"ms_total": ws["merge_ms"], "launches": ws["launches"], "merges": ws["merges"],
+                                    "avg_us": 1e3 * ws["merge_ms"] / ws["launches"], "us_per_merge": 1e3 * ws["merge_ms"] / max(1, ws["merges"]),
+                                    "algorithmic_GB": ws["bytes"] / 1e9, "achieved_GBps": gbs, "frac_of_peak": gbs / peak,
+                                    "dictionary_positions": ws["positions"], "list_entries": ws["list_entries"], "table_scans": ws["table_scans"]}}
+            k = kern["word_merges"]
+            roofline = {"bound": "latency", "kernel": "k_word_merges", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
+                        "peak_source": peak_src, "traffic": None,
+                        "traffic_how": "not captured: a merge touches some hundred records, mostly in L2; dependent round trips and cluster "
+                                       "barriers bound it, not bytes",
+                        "per_launch_algorithmic_bytes": ws["bytes"] / ws["launches"], "avg_launch_us": k["avg_us"], "kernels": kern,
+                        "how": "one extra run with CUDA events around every launch on the library's stream; bytes: occurrence lists read and "
+                               "written, and the scans of the pair table (records and counts of single occurrences not included)"}
+        else:
+            kern = {}
+            for name in ("pair_count", "argmax", "merge_compact"):
+                ms_tot, launches, nb = ks[f"{name}_ms"], ks[f"{name}_launches"], ks[f"{name}_bytes"]
+                gbs = (nb / 1e9) / (ms_tot / 1e3) if ms_tot > 0 else 0.0
+                kern[name] = {"ms_total": ms_tot, "launches": launches, "avg_us": 1e3 * ms_tot / max(1, launches),
+                              "algorithmic_GB": nb / 1e9, "achieved_GBps": gbs, "frac_of_peak": gbs / peak}
+            kern["pair_count"]["skipped_launches"] = ks["pair_count_skipped_launches"]
+            kern["pair_count"]["skipped_ms_total"] = ks["pair_count_skipped_ms"]
+            if world > 1:
+                kern["exchange"] = {"ms_total": ks["exchange_ms"], "launches": ks["exchange_launches"],
+                                    "avg_us": 1e3 * ks["exchange_ms"] / max(1, ks["exchange_launches"]), "kind": exchange}
+            dom = max(("pair_count", "argmax", "merge_compact"), key=lambda k: kern[k]["ms_total"])
+            roofline = {"bound": "hbm", "kernel": "k_" + dom, "achieved": kern[dom]["achieved_GBps"], "peak": peak, "unit": "GB/s",
+                        "frac": kern[dom]["frac_of_peak"], "peak_source": peak_src,
+                        "traffic": NCU_DRAM_PER_ALGORITHMIC_BYTE[dom] * kern[dom]["algorithmic_GB"] * 1e9 / max(1, kern[dom]["launches"]),
+                        "traffic_how": "DRAM read + write bytes per launch: the ncu ratio of DRAM to algorithmic bytes for this kernel "
+                                       "(one capture, summary under profiles/) x the algorithmic bytes of an average launch",
+                        "per_launch_algorithmic_bytes": kern[dom]["algorithmic_GB"] * 1e9 / max(1, kern[dom]["launches"]),
+                        "avg_launch_us": kern[dom]["avg_us"], "kernels": kern,
+                        "how": "one extra run with CUDA events around every kernel on the library's stream (no graph), this rank"}
 
     # ── end to end: host buffers through b200bpe_train, upload and read-back inside the timed region ──
     pin_b = torch.from_numpy(my_data.copy()).pin_memory()

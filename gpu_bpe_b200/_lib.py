@@ -52,6 +52,11 @@ class KernelStats(C.Structure):
                 ("table_update_ms", C.c_double)]
 
 
+class WordStats(C.Structure):
+    _fields_ = [("merge_ms", C.c_double), ("launches", C.c_uint64), ("merges", C.c_uint64), ("positions", C.c_uint64),
+                ("list_entries", C.c_uint64), ("table_scans", C.c_uint64), ("bytes", C.c_uint64)]
+
+
 PROGRESS_CB = C.CFUNCTYPE(None, C.POINTER(Progress), C.c_void_p)
 
 # name → (restype, argtypes); also the list of symbols the header declares
@@ -80,6 +85,7 @@ SIGNATURES = {
     "b200bpe_trainer_kernel_stats": (C.c_int32, [C.c_void_p, C.POINTER(KernelStats)]),
     "b200bpe_trainer_last_run_ms": (C.c_int32, [C.c_void_p, C.POINTER(C.c_double)]),
     "b200bpe_trainer_last_reset_ms": (C.c_int32, [C.c_void_p, C.POINTER(C.c_double)]),
+    "b200bpe_trainer_word_stats": (C.c_int32, [C.c_void_p, C.POINTER(WordStats)]),
     "b200bpe_trainer_launches": (C.c_int32, [C.c_void_p, u64p]),
     "b200bpe_trainer_exchange_kind": (C.c_int32, [C.c_void_p, u32p]),
     "b200bpe_trainer_destroy": (None, [C.c_void_p]),

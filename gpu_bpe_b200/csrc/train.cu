@@ -168,6 +168,8 @@ struct Trainer {
     double last_run_ms = 0, last_reset_ms = 0;
     std::vector<cudaEvent_t> kev;
     b200bpe_kernel_stats stats{};
+    double words_ms = 0;          // of k_word_merges, and its launches, since the last reset
+    uint64_t words_launches = 0;
 
     ~Trainer();
     b200bpe_status alloc_common();
@@ -366,6 +368,8 @@ b200bpe_status Trainer::init_state() {
     early_stop = false;
     cur_n = n0;
     std::memset(&stats, 0, sizeof(stats));
+    words_ms = 0;
+    words_launches = 0;
     by_words = false;
     if (words_eligible()) {
         b200bpe_status r = init_words();
@@ -634,9 +638,9 @@ b200bpe_status Trainer::run_words(uint32_t until, uint32_t start_done, uint32_t*
         if (timed) {
             float ms = 0;
             cudaEventElapsedTime(&ms, kev[0], kev[1]);
-            stats.merge_compact_ms += ms;
-            stats.merge_compact_launches++;
+            words_ms += ms;
         }
+        words_launches++;
         for (uint32_t k = merges_done; k < st.merges_done; k++) {
             const size_t o = (size_t)(k - start_done);
             const uint4 l = w.h_log[k];
@@ -992,17 +996,23 @@ b200bpe_status b200bpe_trainer_pair_counts(b200bpe_trainer* h, uint64_t* keys_ou
         unsigned long long* dk = nullptr;
         uint32_t *dc = nullptr, *dn = nullptr, nd = 0;
         const uint32_t dcap = (uint32_t)std::min<uint64_t>(cap, 1ull << t->words->args.table_log2);
-        B2_CUDA(t->ctx->alloc(&dk, (size_t)dcap * 8));
-        B2_CUDA(t->ctx->alloc(&dc, (size_t)dcap * 4));
-        B2_CUDA(t->ctx->alloc(&dn, 4));
-        B2_CUDA(cudaMemsetAsync(dn, 0, 4, s));
-        k_word_dump<<<t->ctx->sm_count * 4, 256, 0, s>>>(t->words->args.table, t->words->args.table_log2, dk, dc, dcap, dn);
-        B2_CUDA(cudaMemcpyAsync(&nd, dn, 4, cudaMemcpyDeviceToHost, s));
-        B2_CUDA(cudaStreamSynchronize(s));
-        const uint32_t m = std::min(nd, dcap);
-        if (keys_out) B2_CUDA(cudaMemcpy(keys_out, dk, (size_t)m * 8, cudaMemcpyDeviceToHost));
-        if (counts_out) B2_CUDA(cudaMemcpy(counts_out, dc, (size_t)m * 4, cudaMemcpyDeviceToHost));
+        auto dump = [&]() -> b200bpe_status {
+            B2_CUDA(t->ctx->alloc(&dk, (size_t)dcap * 8));
+            B2_CUDA(t->ctx->alloc(&dc, (size_t)dcap * 4));
+            B2_CUDA(t->ctx->alloc(&dn, 4));
+            B2_CUDA(cudaMemsetAsync(dn, 0, 4, s));
+            k_word_dump<<<t->ctx->sm_count * 4, 256, 0, s>>>(t->words->args.table, t->words->args.table_log2, dk, dc, dcap, dn);
+            B2_CUDA(cudaMemcpyAsync(&nd, dn, 4, cudaMemcpyDeviceToHost, s));
+            B2_CUDA(cudaStreamSynchronize(s));
+            const uint32_t m = std::min(nd, dcap);
+            if (keys_out) B2_CUDA(cudaMemcpyAsync(keys_out, dk, (size_t)m * 8, cudaMemcpyDeviceToHost, s));
+            if (counts_out) B2_CUDA(cudaMemcpyAsync(counts_out, dc, (size_t)m * 4, cudaMemcpyDeviceToHost, s));
+            B2_CUDA(cudaStreamSynchronize(s));
+            return B200BPE_OK;
+        };
+        const b200bpe_status r = dump();
         for (void* p : {(void*)dk, (void*)dc, (void*)dn}) t->ctx->free(p);
+        if (r) return r;
         *n_distinct_out = nd;
         return nd > cap ? B200BPE_ERR_CAPACITY : B200BPE_OK;
     }
@@ -1085,6 +1095,22 @@ b200bpe_status b200bpe_trainer_pair_counts(b200bpe_trainer* h, uint64_t* keys_ou
 b200bpe_status b200bpe_trainer_kernel_stats(b200bpe_trainer* h, b200bpe_kernel_stats* out) {
     if (!h || !out) return B200BPE_ERR_BAD_ARG;
     *out = h->t->stats;
+    return B200BPE_OK;
+}
+
+b200bpe_status b200bpe_trainer_word_stats(b200bpe_trainer* h, b200bpe_word_stats* out) {
+    if (!h || !out) return B200BPE_ERR_BAD_ARG;
+    std::memset(out, 0, sizeof(*out));
+    const Trainer& t = *h->t;
+    if (!t.by_words) return B200BPE_OK;
+    const WordState& w = t.words->seen;
+    out->merge_ms = t.words_ms;
+    out->launches = t.words_launches;
+    out->merges = w.merges_done;
+    out->positions = t.words->positions;
+    out->list_entries = w.entries;
+    out->table_scans = w.scans;
+    out->bytes = w.touched + 8ull * w.entries + (uint64_t)w.scans * (16ull << t.words->args.table_log2);
     return B200BPE_OK;
 }
 

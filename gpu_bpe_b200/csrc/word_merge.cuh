@@ -39,6 +39,7 @@ enum : uint32_t { WS_OK = 0, WS_GROW = 1u, WS_FULL = 2u, WS_CAND = 4u, WS_TAIL =
 struct __align__(16) WordState {
     unsigned long long tau;      // threshold of the candidate list, as count << 32 | ~pair; ~0 = no list
     unsigned long long best;     // best pair of the present table, if best_valid
+    unsigned long long touched;  // bytes of occurrence lists and tails that the merges went through (statistics)
     uint32_t best_valid;
     uint32_t merges_done;
     uint32_t next_id;
@@ -161,8 +162,9 @@ struct WordTeam {
 };
 
 // Count updates of up to N pairs by one thread, in step: their probes, insertions and adds are in flight together.  One after the other they
-// were 6,000 of the 10,000 cycles of phase 1, and most of the wait at the barrier behind it: 64 MiB, 8,000 merges 85 -> 65 ms.  wanted: bit k = pair[k] changes by w[k]; rise: bit k = upwards.  `tau` as in
-// WordState; a rise across it makes the slot a candidate of this CTA.
+// were 6,000 of the 10,000 cycles of phase 1, and most of the wait at the barrier behind it: 64 MiB, 8,000 merges 85 -> 65 ms.
+// wanted: bit k = pair[k] changes by w[k]; rise: bit k = upwards.  `tau` as in WordState; a rise across it makes the slot a candidate of
+// this CTA.
 template <int N>
 __device__ __forceinline__ void wt_updates(const WordArgs& A, WordTeam& T, const uint32_t (&pair)[N], const uint32_t (&w)[N], uint32_t wanted, uint32_t rise,
                                            unsigned long long tau) {
@@ -589,7 +591,7 @@ k_word_merges(WordArgs A, uint32_t target) {
     uint32_t done = s.init.merges_done, next_id = s.init.next_id, symbols = s.init.symbols, scans = s.init.scans;
     uint32_t early = s.init.early_stop, status = s.init.status;
     uint32_t front = s.init.front, front_before = s.init.front_before, turn = s.init.turn;
-    unsigned long long tau = s.init.tau, best = s.init.best;
+    unsigned long long tau = s.init.tau, best = s.init.best, touched = s.init.touched;
     bool valid = s.init.best_valid != 0u;
     uint32_t occ_most = s.init.occupied;     // upper bound of the occupied slots
     const uint32_t occ_start = s.init.occupied;
@@ -625,6 +627,7 @@ k_word_merges(WordArgs A, uint32_t target) {
             if (occ_most + grow > room) { status = WS_GROW; break; }
         }
         occ_most += grow;
+        touched += (unsigned long long)len * (bytes ? 4u : 8u) + (LITERAL ? 12ull * (symbols - front) : 0ull);
         TailView tail{};
         uint32_t* tail_src = nullptr;
         uint32_t tail_from = 0u, tail_to = 0u;
@@ -889,6 +892,7 @@ k_word_merges(WordArgs A, uint32_t target) {
         o.occupied = occ_start + s.c_inserted;
         o.symbols = symbols;
         o.scans = scans;
+        o.touched = touched;
         o.front = front;
         o.front_before = front_before;
         o.turn = turn;

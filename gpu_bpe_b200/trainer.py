@@ -128,6 +128,12 @@ class TrainerSession:
         _lib.check(_lib.lib().b200bpe_trainer_kernel_stats(self._h, C.byref(ks)))
         return {f: getattr(ks, f) for f, _ in _lib.KernelStats._fields_}
 
+    def word_stats(self) -> dict:
+        """What training on the dictionary of distinct words took and touched (all 0: the run is on the symbol buffers)."""
+        ws = _lib.WordStats()
+        _lib.check(_lib.lib().b200bpe_trainer_word_stats(self._h, C.byref(ws)))
+        return {f: getattr(ws, f) for f, _ in _lib.WordStats._fields_}
+
     def launches(self) -> int:
         """Kernel launches of this trainer since it was created (a graph launch counts its kernels)."""
         n = C.c_uint64()

@@ -93,7 +93,8 @@ typedef struct {
 } b200bpe_progress;
 typedef void (*b200bpe_progress_cb)(const b200bpe_progress*, void* user);
 
-/* Accumulated device time and algorithmic bytes per kernel class (B200BPE_FLAG_TIME_KERNELS). */
+/* Accumulated device time and algorithmic bytes per kernel class (B200BPE_FLAG_TIME_KERNELS), for the kernels that work on the symbol
+ * buffers; a run on the dictionary of distinct words launches none of them (b200bpe_word_stats). */
 typedef struct {
     double pair_count_ms, argmax_ms, merge_compact_ms, exchange_ms;
     uint64_t pair_count_launches, argmax_launches, merge_compact_launches, exchange_launches;
@@ -106,6 +107,18 @@ typedef struct {
     /* the small kernels that fold the queued pair deltas (and the literal-mode tail) into the table */
     double table_update_ms;
 } b200bpe_kernel_stats;
+
+/* Training on the dictionary of distinct words (one GPU): its merge kernel since the last reset.  All 0 for a run on the symbol buffers. */
+typedef struct {
+    double merge_ms;              /* device time (B200BPE_FLAG_TIME_KERNELS) */
+    uint64_t launches;            /* one per batch of merges, or part of one */
+    uint64_t merges;
+    uint64_t positions;           /* symbols of the distinct words, as bytes */
+    uint64_t list_entries;        /* occurrences of new pairs that were written down */
+    uint64_t table_scans;         /* for a new list of candidates */
+    uint64_t bytes;               /* of what its merges cannot do without: occurrence lists read (4 or 8 bytes an entry) and written (8), the
+                                     tail of a "literal" run read twice and written once, the pair table twice per scan */
+} b200bpe_word_stats;
 
 const char* b200bpe_status_str(b200bpe_status);
 /* Text of the last CUDA/NCCL failure on the calling thread ("" if none). */
@@ -155,11 +168,12 @@ b200bpe_status b200bpe_trainer_run(b200bpe_trainer*, uint32_t max_merges, uint32
 b200bpe_status b200bpe_trainer_reset(b200bpe_trainer*);
 /* Live symbols of this rank (device → host), for tests. */
 b200bpe_status b200bpe_trainer_symbols(b200bpe_trainer*, uint32_t* out, uint64_t cap, uint64_t* n_out);
-/* Run the pair-count kernel on the live symbols and return the table as (a<<32|b, count) entries,
- * unsorted (global counts when sharded); the table is left empty.  For tests. */
+/* The pair counts of the live symbols as (a<<32|b, count) entries, unsorted (global counts when sharded).  A table that is up to date is
+ * read out as it stands; otherwise the pairs are counted now, and the table is left empty.  For tests. */
 b200bpe_status b200bpe_trainer_pair_counts(b200bpe_trainer*, uint64_t* keys_out, uint32_t* counts_out, uint64_t cap,
                                            uint64_t* n_distinct_out);
 b200bpe_status b200bpe_trainer_kernel_stats(b200bpe_trainer*, b200bpe_kernel_stats* out);
+b200bpe_status b200bpe_trainer_word_stats(b200bpe_trainer*, b200bpe_word_stats* out);
 /* Kernels this trainer has launched since it was created (a graph launch counts the kernels it holds);
  * and which count exchange a sharded trainer uses: 0 none (one GPU), 1 peer memory, 2 NCCL.  Diagnostics;
  * no counterpart in the reference. */
