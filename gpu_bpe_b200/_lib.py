@@ -15,7 +15,7 @@ SYNTH_PATH = os.path.join(PKG, "libb200bpe_synth.so")
 u8p, u32p, u64p = C.POINTER(C.c_uint8), C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)
 
 COMPAT_LITERAL, COMPAT_FIXED = 0, 1
-FLAG_NO_GRAPH, FLAG_TIME_KERNELS, FLAG_FULL_RECOUNT, FLAG_NCCL_EXCHANGE = 1, 2, 4, 8
+FLAG_NO_GRAPH, FLAG_TIME_KERNELS, FLAG_FULL_RECOUNT, FLAG_NCCL_EXCHANGE, FLAG_SYMBOL_BUFFERS = 1, 2, 4, 8, 16
 
 STATUS = {0: "OK", 1: "BAD_ARG", 2: "CUDA", 3: "NO_DEVICE", 4: "EMPTY_CORPUS", 5: "TABLE_FULL", 6: "LOOKBACK_TIMEOUT",
           7: "BAD_TRIE_MAGIC", 8: "BAD_TRIE_VERSION", 9: "TRUNCATED_TRIE", 10: "CAPACITY", 11: "NCCL", 12: "OOM",

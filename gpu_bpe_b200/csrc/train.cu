@@ -294,7 +294,7 @@ b200bpe_status Trainer::alloc_common() {
 // Which runs train on the dictionary of distinct words: those on one GPU, new ids above the byte values, no option that
 // is about the other path's kernels (a recount per merge, the test of its bounded wait).  Positions are 32-bit with a bit to spare.
 bool Trainer::words_eligible() const {
-    return !words_refused && ctx->world == 1 && !(opts.flags & B200BPE_FLAG_FULL_RECOUNT) && !opts.test_first_tile &&
+    return !words_refused && ctx->world == 1 && !(opts.flags & (B200BPE_FLAG_FULL_RECOUNT | B200BPE_FLAG_SYMBOL_BUFFERS)) && !opts.test_first_tile &&
            opts.first_token_id >= 256 && n0 < (1ull << 31);
 }
 

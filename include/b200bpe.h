@@ -54,10 +54,12 @@ enum {
     B200BPE_FLAG_FULL_RECOUNT = 4u,  /* rebuild the pair table with a full count before every merge, as the
                                         reference does (train.wgsl:196-202,376-431), instead of updating it in
                                         place around the merged occurrences; the merge list is the same */
-    B200BPE_FLAG_NCCL_EXCHANGE = 8u  /* sharded runs: exchange the pair counts with NCCL send/recv and all-reduce
+    B200BPE_FLAG_NCCL_EXCHANGE = 8u, /* sharded runs: exchange the pair counts with NCCL send/recv and all-reduce
                                         instead of this library's own kernels over NVLink peer memory (the default,
                                         which needs one process per GPU and CUDA IPC between them; the library falls
                                         back to NCCL by itself when the peers' buffers cannot be mapped) */
+    B200BPE_FLAG_SYMBOL_BUFFERS = 16u /* one GPU: train on the symbol buffers, as sharded runs do, also where the dictionary of distinct
+                                        words would take the text; the merge list is the same */
 };
 
 typedef struct b200bpe_ctx b200bpe_ctx;
