@@ -792,13 +792,15 @@ struct Tokenizer {
         return B200BPE_OK;
     }
 
-    b200bpe_status ensure_work(uint64_t max_chunks, bool staging) {
+    // Tiles of the look-back at most: a tile takes whole chunks, SC_THREADS of them, or as many as a CTA of the split walk has threads for.
+    uint64_t most_tiles(uint64_t max_chunks, bool split) const { return max_chunks / (split ? split_threads() / blocks_per_chunk() : SC_THREADS) + 2; }
+
+    b200bpe_status ensure_work(uint64_t max_chunks, bool staging, uint64_t tiles) {
         b200bpe_status r;
         if (staging && (r = ensure(&d_staging, &staging_cap, max_chunks * chunk))) return r;
         if ((r = ensure(&d_counts, &counts_cap, max_chunks + 1))) return r;
         if ((r = ensure(&d_chunk_off, &chunk_off_cap, max_chunks + 1))) return r;
-        // (a tile of the split walk holds one chunk at least)
-        return ensure(&d_desc, &desc_cap, CTL_WORDS + max_chunks + 2);
+        return ensure(&d_desc, &desc_cap, CTL_WORDS + tiles);
     }
 
     size_t walk_smem() const { return hybrid ? (size_t)HY_SMEM_BYTES : ck_d == 0 ? (size_t)TW_SMEM_BYTES : ((size_t)ck_d << ck_log2) * 4; }
@@ -890,9 +892,9 @@ struct Tokenizer {
         if (ck_d == 0 && !hybrid) set_persisting_window(ctx, d_trans, trans_bytes);  // keep the transition table resident in L2
         const uint64_t max_chunks = (n + chunk - 1) / chunk + (d_docs ? n_docs : 0);
         const bool split = split_pays(n, max_chunks);
-        b200bpe_status r = ensure_work(std::max<uint64_t>(1, max_chunks), !split);
+        const uint64_t ntiles = most_tiles(max_chunks, split);
+        b200bpe_status r = ensure_work(std::max<uint64_t>(1, max_chunks), !split, ntiles);
         if (r) return r;
-        const uint64_t ntiles = max_chunks / (split ? split_threads() / blocks_per_chunk() : SC_THREADS) + 2;
         uint64_t* d_total = reinterpret_cast<uint64_t*>(d_desc);
         uint32_t* d_ctl = reinterpret_cast<uint32_t*>(d_desc + 1);
         unsigned long long* desc = d_desc + CTL_WORDS;
@@ -1448,7 +1450,7 @@ b200bpe_status b200bpe_encode_batch(b200bpe_tok* h, const uint8_t* bytes, const 
     if ((r = t->ensure(&t->d_tok_off, &t->tok_off_cap, (uint64_t)n_docs + n_slices + 1))) return r;
     // document offsets relative to the first byte of their slice, one run of (docs + 1) entries per slice
     std::vector<uint64_t> rel((size_t)n_docs + n_slices);
-    uint64_t max_chunks = 1;
+    uint64_t max_chunks = 1, max_tiles = 1;
     uint32_t max_docs = 1;
     bool staging = false;
     for (uint32_t i = 0; i < n_slices; i++) {
@@ -1456,11 +1458,13 @@ b200bpe_status b200bpe_encode_batch(b200bpe_tok* h, const uint8_t* bytes, const 
         for (uint32_t d = d0; d <= d1; d++) rel[(size_t)d + i] = doc_offsets[d] - doc_offsets[d0];
         const uint64_t nb = doc_offsets[d1] - doc_offsets[d0], chunks = (nb + t->chunk - 1) / t->chunk + (d1 - d0);
         max_chunks = std::max<uint64_t>(max_chunks, chunks);
-        staging |= !t->split_pays(nb, chunks);
+        const bool split = t->split_pays(nb, chunks);
+        staging |= !split;
+        max_tiles = std::max(max_tiles, t->most_tiles(chunks, split));
         max_docs = std::max(max_docs, d1 - d0);
     }
     // every buffer a slice needs exists before the first one starts (growing one synchronises the stream)
-    if ((r = t->ensure_work(max_chunks, staging))) return r;
+    if ((r = t->ensure_work(max_chunks, staging, max_tiles))) return r;
     if ((r = t->ensure(&t->d_chunk_base, &t->chunk_base_cap, (uint64_t)max_docs + 1))) return r;
     if ((r = t->ensure_slices(n_slices))) return r;
     B2_CUDA(cudaMemcpyAsync(t->d_doc_off, rel.data(), rel.size() * 8, cudaMemcpyHostToDevice, s));

@@ -96,3 +96,21 @@ def test_a_small_vocabulary_beside_a_large_one(engine, layout):
         assert t.encodeBytes(large).size == O.encode(large, trie, t.chunkSize).size, n
     for t in toks:
         t.destroy()
+
+
+@pytest.mark.parametrize("layout", ["auto", "hybrid"])
+def test_one_handle_for_both_walks(engine, layout):
+    """Sizes that go through either walk in turn on one handle, whose look-back descriptors grow with the tiles of the walk that runs."""
+    data = np.tile(_runs(np.random.default_rng(5), 1 << 20), 60)
+    trie = compileVocabToTrie(RUNS)
+    one, sliced = (TrieTokenizer(engine, trie, RUNS, {"layout": layout, **o}) for o in ({}, {"encodeSliceBytes": 1 << 20}))
+    for n in (60 << 20, 100, 5_000_001, 30 << 20, 60 << 20):
+        assert np.array_equal(one.encodeBytes(data[:n]), sliced.encodeBytes(data[:n])), n
+    fresh = TrieTokenizer(engine, trie, RUNS, {"layout": layout, "batchSliceBytes": 1 << 20})
+    for docs in (40, 30_000, 7):              # slices of a batch that take different walks: few long documents, then many short ones
+        offs = np.unique(np.concatenate([[0, 6 << 20, 12 << 20], (6 << 20) + np.arange(docs) * 200])).astype(np.uint64)
+        got, toff = fresh.encodeBatch(data[:12 << 20], offs)
+        want, woff = O.encode_batch(data[:12 << 20], offs, trie, fresh.chunkSize)
+        assert np.array_equal(got, want) and np.array_equal(toff, woff), docs
+    for t in (one, sliced, fresh):
+        t.destroy()
