@@ -32,6 +32,17 @@ b200bpe_status load_nccl(const char* path, NcclApi* api) {
     return B200BPE_OK;
 }
 
+static void let_go(b200bpe_ctx* c) {
+    if (c->c.holders.fetch_sub(1) != 1) return;
+    cudaSetDevice(c->c.device);
+    if (c->c.stream) cudaStreamDestroy(c->c.stream);
+    if (c->c.pool) cudaMemPoolDestroy(c->c.pool);
+    for (const auto& b : c->c.pinned) cudaFreeHost(b.p);
+    delete c;
+}
+void CtxHold::take(b200bpe_ctx* c) { held = c; c->c.holders.fetch_add(1); }
+CtxHold::~CtxHold() { if (held) let_go(held); }
+
 static b200bpe_status make_ctx(int device, b200bpe_ctx** out) {
     if (!out) return B200BPE_ERR_BAD_ARG;
     int count = 0;
@@ -144,10 +155,8 @@ void b200bpe_ctx_destroy(b200bpe_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->c.device);
     if (c->c.comm && c->c.nccl.CommDestroy) c->c.nccl.CommDestroy(c->c.comm);
-    if (c->c.stream) cudaStreamDestroy(c->c.stream);
-    if (c->c.pool) cudaMemPoolDestroy(c->c.pool);
-    for (const auto& b : c->c.pinned) cudaFreeHost(b.p);
-    delete c;
+    c->c.comm = nullptr;
+    let_go(c);
 }
 
 b200bpe_status b200bpe_ctx_info(b200bpe_ctx* c, int32_t* sm_count, int32_t* cc, uint64_t* total_mem, uint64_t* free_mem) {

@@ -1,6 +1,7 @@
 // Context object: one GPU, one stream, optional NCCL communicator for sharded jobs.
 #pragma once
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -27,6 +28,7 @@ struct NcclApi {
     const char* (*GetErrorString)(int) = nullptr;
 };
 struct Ctx {
+    std::atomic<uint32_t> holders{1};    // its creator, and every handle made with it
     int device = 0;
     cudaStream_t stream = nullptr;
     int sm_count = 0;
@@ -81,6 +83,14 @@ struct Ctx {
         }
         cudaFreeHost(p);
     }
+};
+
+// A handle's share of its context.  Handles give their memory back to the context's pool on its stream, so both stay until the last
+// handle is gone, whichever order the caller destroys them in.  Declared first in a handle: it goes after everything else.
+struct CtxHold {
+    b200bpe_ctx* held = nullptr;
+    void take(b200bpe_ctx* c);
+    ~CtxHold();
 };
 
 b200bpe_status load_nccl(const char* path, NcclApi* api);

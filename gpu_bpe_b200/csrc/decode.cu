@@ -87,6 +87,7 @@ k_decode_copy(const uint32_t* __restrict__ tokens, uint64_t n, const uint64_t* _
 }
 
 struct Decoder {
+    CtxHold hold;
     Ctx* ctx = nullptr;
     cudaStream_t stream = nullptr;
     uint32_t entries = 0;
@@ -186,6 +187,7 @@ b200bpe_status b200bpe_decoder_create(b200bpe_ctx* c, const uint8_t* bytes, cons
     b200bpe_decoder* h = new b200bpe_decoder();
     Decoder& d = h->d;
     d.ctx = &c->c;
+    d.hold.take(c);
     d.entries = n_entries;
     static const uint8_t replacement[3] = {0xEF, 0xBF, 0xBD};
     const uint64_t end = n + 3;

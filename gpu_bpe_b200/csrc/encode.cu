@@ -727,6 +727,7 @@ static cudaError_t allow_all_shared_memory(Kernel* kernel) {
 }
 
 struct Tokenizer {
+    CtxHold hold;
     Ctx* ctx = nullptr;
     uint32_t node_count = 0, edge_count = 0, max_token_len = 0, chunk = 0;
     uint2* d_trans = nullptr;      // large tries: global transition table
@@ -1286,6 +1287,7 @@ b200bpe_status b200bpe_tokenizer_create_ex(b200bpe_ctx* c, const void* trie, siz
     B2_CUDA(cudaSetDevice(c->c.device));
     Tokenizer* t = new Tokenizer();
     t->ctx = &c->c;
+    t->hold.take(c);
     t->node_count = node_count; t->edge_count = edge_count; t->max_token_len = max_len;
     t->chunk = chunk_size ? chunk_size : std::max(512u, std::min(2048u, max_len * 8u));  // tokenizer.js:67-68
     t->trans_mask = tmask;

@@ -474,6 +474,7 @@ k_replay_segments(SegmentState* __restrict__ st, const uint8_t* __restrict__ byt
 }
 
 struct Replay {
+    CtxHold hold;
     Ctx* ctx = nullptr;
     uint32_t n_rules = 0;
     uint32_t* d_rules = nullptr;
@@ -689,6 +690,7 @@ b200bpe_status b200bpe_replay_create(b200bpe_ctx* c, const uint32_t* merges, uin
     B2_CUDA(cudaSetDevice(c->c.device));
     Replay* rp = new Replay();
     rp->ctx = &c->c;
+    rp->hold.take(c);
     rp->n_rules = n_merges;
     auto fail = [&](b200bpe_status st) { delete rp; return st; };
     uint32_t lg = 4;

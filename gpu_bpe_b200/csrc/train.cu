@@ -119,6 +119,7 @@ static b200bpe_status agree_on_max(Ctx* ctx, unsigned long long* v) {
 }
 
 struct Trainer {
+    CtxHold hold;
     Ctx* ctx = nullptr;
     uint64_t n0 = 0;            // symbols at creation (this rank)
     b200bpe_train_opts opts{};
@@ -881,6 +882,7 @@ static b200bpe_status make_trainer(b200bpe_ctx* c, const uint8_t* bytes, const u
     B2_CUDA(cudaSetDevice(c->c.device));
     Trainer* t = new Trainer();
     t->ctx = &c->c;
+    t->hold.take(c);
     t->n0 = n;
     b200bpe_status r = check_opts(&c->c, opts, &t->opts);
     if (r) { delete t; return r; }

@@ -159,8 +159,7 @@ class TrieTokenizer:
 
     def destroy(self):
         with self._decode_lock:
-            if self._engine._ctx is not None:
-                self._drop_decoder()
+            self._drop_decoder()
         if self._h is not None:
             _lib.lib().b200bpe_tokenizer_destroy(self._h)
             self._h = None

@@ -136,6 +136,7 @@ b200bpe_status b200bpe_ctx_create(int32_t device, b200bpe_ctx** out);
 b200bpe_status b200bpe_nccl_unique_id(const char* nccl_lib, uint8_t unique_id[128]);
 b200bpe_status b200bpe_ctx_create_dist(int32_t device, int32_t rank, int32_t world, const char* nccl_lib,
                                        const uint8_t unique_id[128], b200bpe_ctx** out);
+/* Handles made with the context may be destroyed before it or after it. */
 void b200bpe_ctx_destroy(b200bpe_ctx*);
 /* Device facts: sm_count, compute capability major*10+minor, total and free memory in bytes. */
 b200bpe_status b200bpe_ctx_info(b200bpe_ctx*, int32_t* sm_count, int32_t* cc, uint64_t* total_mem, uint64_t* free_mem);
