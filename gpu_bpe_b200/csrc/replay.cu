@@ -304,7 +304,7 @@ k_replay_segments(SegmentState* __restrict__ st, const uint8_t* __restrict__ byt
                   unsigned long long* __restrict__ desc, uint32_t* __restrict__ out) {
     __shared__ uint32_t tok[RS_SPAN], rnk[RS_SPAN];     // rnk[i]: rank of the rule for tokens i and i + 1 of the same segment
     __shared__ uint16_t start[RS_TILE], cnt[RS_TILE], longs[RS_TILE / RS_SHORT + 1];
-    __shared__ uint32_t s_tile, s_warp[RS_THREADS / 32], s_next, s_longs, s_excl;
+    __shared__ uint32_t s_tile, s_warp[RS_THREADS / 32], s_next, s_longs, s_excl, s_over;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ntiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
     auto ranks2 = [&](unsigned long long p0, unsigned long long p1, uint32_t& r0, uint32_t& r1) {
@@ -315,7 +315,7 @@ k_replay_segments(SegmentState* __restrict__ st, const uint8_t* __restrict__ byt
     };
     for (;;) {
         __syncthreads();
-        if (tid == 0) { s_tile = atomicAdd(&st->ticket, 1u); s_longs = 0u; }
+        if (tid == 0) { s_over = *reinterpret_cast<volatile uint32_t*>(&st->status); s_tile = atomicAdd(&st->ticket, 1u); s_longs = 0u; }
         __syncthreads();
         const uint32_t tile = s_tile;
         if (tile >= ntiles) return;
@@ -363,8 +363,14 @@ k_replay_segments(SegmentState* __restrict__ st, const uint8_t* __restrict__ byt
         uint32_t end = s_next;               // of the last segment that begins here
         if (end == RS_NONE || end > (uint32_t)(RS_TILE + RS_HALO)) {
             end = RS_TILE + RS_HALO;
-            if (tid == 0 && segments) atomicMax(&st->status, 1u);
+            if (segments) {
+                if (tid == 0) atomicMax(&st->status, 1u);
+                segments = 0u;
+            }
         }
+        // A text with a segment too long goes through the rounds: nothing that is left is worth doing but to tell the tiles behind that
+        // there are no tokens here.
+        if (s_over) segments = 0u;
         __syncthreads();
         // the byte pairs' ranks
         if (segments) {
@@ -406,31 +412,49 @@ k_replay_segments(SegmentState* __restrict__ st, const uint8_t* __restrict__ byt
         for (uint32_t q = warp; q < s_longs; q += RS_THREADS / 32) {
             const uint32_t i = longs[q], s = start[i];
             uint32_t m = (i + 1u < segments ? start[i + 1] : end) - s;
+            // A pass applies all pairs of the smallest rank, from the left, as a rule does: in a run of matches (of two equal tokens) every other
+            // one.  A segment of a repeated byte then takes as many passes as rules apply, not a step per token (1,536 x "a": a call 2.0 -> 0.11 ms, in rounds 0.27).
+            uint32_t best = RS_NONE;
+            for (uint32_t j = lane; j + 1u < m; j += 32) best = min(best, rnk[s + j]);
             for (;;) {
-                uint32_t best = RS_NONE, b = 0u;
-                for (uint32_t j = lane; j + 1u < m; j += 32) { const uint32_t r = rnk[s + j]; if (r < best) { best = r; b = j; } }
                 const uint32_t all = __reduce_min_sync(0xFFFFFFFFu, best);
                 if (all == RS_NONE) break;
-                b = __reduce_min_sync(0xFFFFFFFFu, best == all ? b : RS_NONE);
-                const uint32_t t = 256u + all;
-                for (uint32_t j0 = b + 1u; j0 + 1u < m; j0 += 32) {
+                const uint32_t t = 256u + all, below = (1u << lane) - 1u;
+                uint32_t kept = 0u, odd = 0u, drop = 0u;     // of the block before: its last run of matches has an odd length; its last token is taken
+                for (uint32_t j0 = 0u; j0 < m; j0 += 32) {
                     const uint32_t j = j0 + lane;
-                    const bool in = j + 1u < m;
-                    const uint32_t a = in ? tok[s + j + 1] : 0u, r = in ? rnk[s + j + 1] : 0u;
-                    __syncwarp();
-                    if (in) { tok[s + j] = a; rnk[s + j] = r; }
-                    __syncwarp();
+                    const uint32_t a = j < m ? tok[s + j] : 0u, r = j + 1u < m ? rnk[s + j] : RS_NONE;
+                    const uint32_t match = __ballot_sync(0xFFFFFFFFu, r == all);
+                    const uint32_t gap = ~match & below;     // lanes below this one without a match
+                    const uint32_t place = gap ? lane - (32u - (uint32_t)__clz((int)gap)) : lane + odd;   // in the run of matches
+                    const bool take = r == all && !(place & 1u);
+                    const uint32_t taken = __ballot_sync(0xFFFFFFFFu, take);
+                    const bool keep = j < m && !((taken << 1 | drop) >> lane & 1u);
+                    const uint32_t keeps = __ballot_sync(0xFFFFFFFFu, keep);
+                    __syncwarp();                            // everybody has read the block
+                    if (keep) {
+                        const uint32_t p = s + kept + (uint32_t)__popc(keeps & below);
+                        tok[p] = take ? t : a;
+                        rnk[p] = r;
+                    }
+                    kept += (uint32_t)__popc(keeps);
+                    odd = match == 0xFFFFFFFFu ? odd : (uint32_t)__clz((int)~match) & 1u;   // (a whole block of matches is an even number)
+                    drop = taken >> 31;
                 }
-                m--;
-                if (lane == 0) { applied[all] = 1; tok[s + b] = t; }
+                m = kept;
+                if (lane == 0) applied[all] = 1;
                 __syncwarp();
-                if (lane < 2u) {
-                    const bool left = lane == 0;
-                    const bool there = left ? b > 0u : b + 1u < m;
-                    const unsigned long long p = left ? rs_pair(there ? tok[s + b - 1] : 0x1FFFFFu, t) : rs_pair(t, there ? tok[s + b + 1] : 0x1FFFFFu);
-                    const uint32_t slot = rs_hash(p) & R.mask;
-                    const uint32_t r = rs_rank(R, p, slot, __ldg(R.table + slot));
-                    if (there || !left) rnk[left ? s + b - 1 : s + b] = r;
+                best = RS_NONE;                              // the ranks beside the new tokens, and the smallest of all
+                for (uint32_t j = lane; j + 1u < m; j += 32) {
+                    const uint32_t x = tok[s + j], y = tok[s + j + 1];
+                    uint32_t r = rnk[s + j];
+                    if (x == t || y == t) {
+                        const unsigned long long p = rs_pair(x, y);
+                        const uint32_t slot = rs_hash(p) & R.mask;
+                        r = rs_rank(R, p, slot, __ldg(R.table + slot));
+                        rnk[s + j] = r;
+                    }
+                    best = min(best, r);
                 }
                 __syncwarp();
             }

@@ -41,3 +41,27 @@ def test_a_handle_takes_texts_with_and_without_long_segments_in_turn(engine):
         data = _text(rng, lengths, n)
         assert np.array_equal(tm.encodeBytes(data), O.replay_encode(data, RULES))
     tm.destroy()
+
+
+@pytest.mark.parametrize("length", [33, 34, 63, 64, 65, 95, 96, 97, 500, 1000, 1400, 1535])
+@pytest.mark.parametrize("kind", ["a", "ab", "aab", "two letters", "runs"])
+def test_long_segments_of_few_letters(engine, length, kind):
+    """Pairs of equal tokens in runs either side of a warp's 32 tokens, whose every other one is taken, from the left; several of them a tile."""
+    rng = np.random.default_rng(length)
+    rules = [[97, 97, 300], [300, 300, 301], [301, 301, 302], [97, 98, 303], [303, 303, 304], [98, 98, 305], [305, 305, 306], [300, 98, 307],
+             [98, 300, 308], [304, 304, 309], [302, 97, 310], [309, 97, 311], [305, 97, 312], [306, 306, 313], [302, 302, 314]]
+    parts = []
+    for k in range(12):
+        m = max(1, length - int(rng.integers(0, 3)) if k % 3 else length)
+        if kind == "two letters":
+            w = 97 + rng.integers(0, 2, m)
+        elif kind == "runs":
+            w = np.concatenate([np.full(int(rng.integers(1, 80)), 97 + k % 2 if rng.random() < 0.8 else 98) for _ in range(m)])[:m]
+        else:
+            w = np.resize(np.frombuffer(kind.encode(), np.uint8), m)
+        parts += [w.astype(np.uint8), np.full(int(rng.integers(1, 40)), 46, np.uint8)]
+    for data in (np.concatenate(parts), parts[0], np.concatenate(parts[:3])):
+        for use in (rules, rules[:1], rules[:4]):
+            tm = TokenizerManager(engine, {"merges": use})
+            assert np.array_equal(tm.encodeBytes(data), O.replay_encode(data, use)), (len(use), data.size)
+            tm.destroy()
