@@ -38,19 +38,54 @@ struct Ctx {
     void* comm = nullptr;
     // Device memory of this context's short-lived objects, in the order of a stream (its own, or that of an object with one): an allocation is a few microseconds when
     // the pool has the block, against hundreds for cudaMalloc.  At most POOL_KEEP bytes stay with the pool between calls; the
-    // rest goes back to the device at the next synchronisation, and all of it with the context.
+    // rest goes back to the device at the next synchronisation, and all of it with the context.  Blocks of more than POOL_BLOCK bytes are
+    // not the pool's: it could not keep them, and maps and unmaps 10 GB in 50 ms each (at times ten times that), cudaMalloc and
+    // cudaFree in 5 and 12.
     cudaMemPool_t pool = nullptr;
     static constexpr unsigned long long POOL_KEEP = 2ull << 30;
+    static constexpr size_t POOL_BLOCK = 512ull << 20;
+    std::vector<void*> large;
+    std::mutex large_mutex;
     template <class T>
     cudaError_t alloc(T** p, size_t bytes, cudaStream_t on) {
         void* v = nullptr;
-        const cudaError_t e = cudaMallocFromPoolAsync(&v, bytes ? bytes : 1, pool, on);
+        cudaError_t e;
+        if (bytes <= POOL_BLOCK) {
+            e = cudaMallocFromPoolAsync(&v, bytes ? bytes : 1, pool, on);
+        } else {
+            e = cudaMalloc(&v, bytes);
+            if (e == cudaErrorMemoryAllocation) {        // (what the pool keeps may be what is missing)
+                cudaGetLastError();
+                cudaStreamSynchronize(on);
+                cudaMemPoolTrimTo(pool, 0);
+                e = cudaMalloc(&v, bytes);
+            }
+            if (e == cudaSuccess) {
+                std::lock_guard<std::mutex> lock(large_mutex);
+                large.push_back(v);
+            }
+        }
         *p = static_cast<T*>(v);
         return e;
     }
     template <class T>
     cudaError_t alloc(T** p, size_t bytes) { return alloc(p, bytes, stream); }
-    void free(void* p, cudaStream_t on) { if (p) cudaFreeAsync(p, on); }
+    void free(void* p, cudaStream_t on) {
+        if (!p) return;
+        {
+            std::unique_lock<std::mutex> lock(large_mutex);
+            for (size_t i = 0; i < large.size(); i++)
+                if (large[i] == p) {
+                    large[i] = large.back();
+                    large.pop_back();
+                    lock.unlock();
+                    cudaStreamSynchronize(on);           // (a pool's block may still be in use by what is enqueued; so may this one)
+                    cudaFree(p);
+                    return;
+                }
+        }
+        cudaFreeAsync(p, on);
+    }
     void free(void* p) { free(p, stream); }
     // Pinned host memory of this context's short-lived objects: cudaMallocHost takes 3 to 5 ms, half of a training call on a page of
     // text.  A few blocks are kept between objects, PINNED_KEEP bytes at most, and go with the context.  A block is only given back when no
