@@ -3,9 +3,9 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--config 3]
 
 Default workload (config 3 of the benchmark list): train 32,000 merges on 1 GiB of seeded synthetic
-UTF-8 text.  One step = one complete training run on the HBM-resident corpus: re-tag the symbols,
-then the whole merge loop (250 CUDA-graph launches of 128 merges, one read-back each).  N > 1 (under
-torchrun): the same corpus cut at word starts across the ranks, "fixed" compaction mode, the pair
+UTF-8 text.  One step = one complete training run on the HBM-resident corpus: set the
+state up from the resident bytes, then the whole merge loop (250 launches of 128 merges, one read-back
+each).  N > 1 (under torchrun): the same corpus cut at word starts across the ranks, "fixed" compaction mode, the pair
 counts exchanged by this library's kernels over NVLink peer memory (strong scaling).  The merge list
 and its counts are compared, all 32,000 entries, with the golden list of tests/golden/.
 

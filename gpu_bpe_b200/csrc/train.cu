@@ -1,6 +1,6 @@
-// Host side of the training path: device buffers, the per-batch CUDA graph, the batch loop
-// that mirrors BPETrainer.#runTrainingLoop (src/bpe/trainer.js:225-335 of the reference), and
-// the C entry points declared in include/b200bpe.h.
+// Host side of the training path: the choice between the dictionary of distinct words (word_path.cuh) and the symbol buffers; these
+// buffers, their per-batch CUDA graph, the batch loops that mirror BPETrainer.#runTrainingLoop (src/bpe/trainer.js:225-335 of the
+// reference), and the C entry points declared in include/b200bpe.h.
 #include <algorithm>
 #include <chrono>
 #include <cstdio>

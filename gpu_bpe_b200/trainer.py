@@ -3,7 +3,7 @@
 Mirrors BPETrainer of src/bpe/trainer.js:125-371 of the reference: the same constructor, the
 same train(input, {targetVocabSize, preTokenizer, onProgress}) arguments and result object, the
 same error for an empty corpus, the same progress payload.  The merge loop itself runs in
-libb200bpe.so (128 merges per CUDA-graph launch, one read-back per batch).
+libb200bpe.so (128 merges per launch, one read-back per batch).
 """
 from __future__ import annotations
 
