@@ -33,6 +33,7 @@ struct DictState {
     uint32_t words;          // distinct words
     uint32_t pairs;          // distinct byte pairs
     unsigned long long split;   // "literal" runs: where the tail begins
+    unsigned long long sampled, squares;   // of a sample of byte pairs: their number, and the sum of the squares of each pair's
 };
 
 struct DictTables {
@@ -475,6 +476,27 @@ k_dict_tail(const uint8_t* __restrict__ bytes, const uint8_t* __restrict__ mask,
         const uint32_t r = bytes[i + 1];
         if (l && r) atomicAdd(bins + (l << 8 | r), 1ull);
     }
+}
+
+// ── how many byte pairs a text uses ──
+// A place in each of WD_SAMPLE equal parts of the text (scattered, so that no column of a table is all there is): the pairs of different
+// bytes there, inside words, counted in the bins.  A pair of equal bytes does not count, because a run of them is gone with one merge.  One CTA.
+constexpr uint32_t WD_SAMPLE = 32768;
+__global__ void __launch_bounds__(1024)
+k_dict_sample(const uint8_t* __restrict__ bytes, const uint8_t* __restrict__ mask, uint64_t n, unsigned long long* __restrict__ bins, DictState* __restrict__ st) {
+    const uint64_t step = n / WD_SAMPLE + 1;
+    unsigned long long squares = 0ull, taken = 0ull;
+#pragma unroll 8
+    for (uint32_t k = threadIdx.x; k < WD_SAMPLE; k += 1024) {
+        const uint64_t i = k * step + k * 0x9E3779B1u % step;
+        if (i + 1 >= n || mask[i + 1]) continue;
+        const uint32_t l = bytes[i], r = bytes[i + 1];
+        if (l == r || l == 0u || r == 0u) continue;
+        squares += 2ull * atomicAdd(bins + (l << 8 | r), 1ull) + 1ull;      // (k + 1)^2 - k^2
+        taken++;
+    }
+    atomicAdd(&st->squares, squares);
+    atomicAdd(&st->sampled, taken);
 }
 
 // ── the live symbols, in text order ──

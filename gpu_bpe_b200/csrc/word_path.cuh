@@ -2,6 +2,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -106,6 +107,23 @@ struct WordPath {
     uint64_t tail_goal() const { return n / 32 * tail_share; }
     int aligned() const { return (((uintptr_t)bytes | (uintptr_t)mask) & 15u) == 0 ? 1 : 0; }
 
+    // Texts of few letters whose words are mostly distinct (DNA, digits) are the symbol buffers': a merge then has millions of occurrences in
+    // the dictionary too, on 16 SMs and with their counts on a few hot slots.  With P positions for n bytes and E byte pairs in use (the
+    // inverse of the chance that two pairs are the same), merges with the dictionary took 10 P / (n sqrt E) times as long as on the symbol
+    // buffers where these merges are most of a run, and what later merges save pays for 3,500 of P / sqrt E each; in "literal" runs an
+    // explicit symbol of the tail costs as much as two positions, and a later merge saves a quarter of that.  Create + run, dictionary / symbol
+    // buffers, ms, 128 MiB of distinct words of 65 letters, 64 merges: 2 letters 324 / 61, 4 letters 231 / 90, 8 letters 135 / 97, 12 letters
+    // 103 / 102, 64 letters 47 / 61; 4 letters, 4,000 merges 568 / 480, every word four times 170 / 466.  Up to 4 MiB the dictionary was never
+    // slower.  A text that goes to the symbol buffers by this rule pays 1 ms per 128 MiB for having its words looked up.
+    static constexpr uint64_t FEW_LETTERS_FROM = 8ull << 20;
+    bool few_letters() const {
+        if (h_dict->squares == 0) return false;
+        const double e = (double)h_dict->sampled * (double)h_dict->sampled / (double)h_dict->squares;
+        // (a first merge of more than a 32nd of the text needs the long tail)
+        const double tail = literal ? (double)n / 32 * (e < 32 ? TAIL_LONG : tail_share) : 0.0;
+        return ((double)h_dict->positions + 2 * tail) / std::sqrt(e) > (double)n / 10 + (literal ? 900.0 : 3500.0) * goal;
+    }
+
     // Builds the dictionary of the text and the state of a fresh run.  *fits is false (and nothing else is set up) when the text is
     // not one of words that a dictionary pays for: the symbol buffers of the other path then take it.
     b200bpe_status build(const uint8_t* d_bytes, const uint8_t* d_mask, const uint32_t* d_symbols, uint32_t first_id, bool* fits) {
@@ -140,6 +158,12 @@ struct WordPath {
             n_front = h_dict->split;
             if (n_front == 0 || n_front >= n) return B200BPE_OK;
         }
+        const bool large = n_front >= FEW_LETTERS_FROM;
+        if (large) {
+            B2_CUDA(cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 65536, s));
+            k_dict_sample<<<1, 1024, 0, s>>>(bytes, mask, n_front, bins, dict.st);
+            launches++;
+        }
         k_dict_words<<<blocks(n_front, WD_TILE, 3), WD_THREADS, WD_SMEM_BYTES, s>>>(bytes, mask, n_front, dict, aligned());
         const uint64_t slots = (1ull << dict.short_log2) + (1ull << dict.long_log2);
         k_dict_places<<<blocks(slots, 1024, 8), 256, 0, s>>>(mask, n_front, dict);
@@ -147,7 +171,7 @@ struct WordPath {
         B2_CUDA(cudaMemcpyAsync(h_dict, dict.st, sizeof(DictState), cudaMemcpyDeviceToHost, s));
         B2_CUDA(cudaStreamSynchronize(s));
         B2_CUDA(cudaGetLastError());
-        if (h_dict->status) return B200BPE_OK;
+        if (h_dict->status || (large && few_letters())) return B200BPE_OK;
         positions = h_dict->positions;
         args.positions = positions;
         if (positions > cap_positions || !args.rec) {
