@@ -35,7 +35,7 @@ b200bpe_status load_nccl(const char* path, NcclApi* api) {
 static void let_go(b200bpe_ctx* c) {
     if (c->c.holders.fetch_sub(1) != 1) return;
     cudaSetDevice(c->c.device);
-    if (c->c.stream) cudaStreamDestroy(c->c.stream);
+    for (cudaStream_t s : {c->c.stream, c->c.decode_stream}) if (s) cudaStreamDestroy(s);
     if (c->c.pool) cudaMemPoolDestroy(c->c.pool);
     for (const auto& b : c->c.pinned) cudaFreeHost(b.p);
     delete c;
@@ -64,6 +64,7 @@ static b200bpe_status make_ctx(int device, b200bpe_ctx** out) {
     c->c.sm_count = prop.multiProcessorCount;
     c->c.cc = prop.major * 10 + prop.minor;
     cudaError_t e = cudaStreamCreateWithFlags(&c->c.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->c.decode_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;

@@ -31,12 +31,13 @@ struct Ctx {
     std::atomic<uint32_t> holders{1};    // its creator, and every handle made with it
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t decode_stream = nullptr;   // the decoders': any thread may use it, and nobody records a graph from it
     int sm_count = 0;
     int cc = 0;
     int rank = 0, world = 1;
     NcclApi nccl;
     void* comm = nullptr;
-    // Device memory of this context's short-lived objects, in the order of a stream (its own, or that of an object with one): an allocation is a few microseconds when
+    // Device memory of this context's short-lived objects, in the order of one of its streams: an allocation is a few microseconds when
     // the pool has the block, against hundreds for cudaMalloc.  At most POOL_KEEP bytes stay with the pool between calls; the
     // rest goes back to the device at the next synchronisation, and all of it with the context.  Blocks of more than POOL_BLOCK bytes are
     // not the pool's: it could not keep them, and maps and unmaps 10 GB in 50 ms each (at times ten times that), cudaMalloc and
